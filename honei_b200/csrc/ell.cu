@@ -316,7 +316,7 @@ namespace hb2
 
     // HB2_Q1_TRANSFER=0 runs the Q1 transfer matrices on their stored layout instead
     // (read at every launch, so a process can compare both)
-    static bool q1_transfer_kernels_enabled()
+    bool q1_transfer_kernels_enabled()
     {
         const char * v = getenv("HB2_Q1_TRANSFER");
         return ! (v && strcmp(v, "0") == 0);
@@ -921,6 +921,29 @@ extern "C" int hb2_jacobi_ell(hb2_ell A, const void * P, const void * b, void * 
 {
     if (! A || ! P || ! b || ! x || (sweeps > 0 && ! tmp)) return fail(HB2_ERR_ARG, "hb2_jacobi_ell: null argument");
     if (A->rows != A->cols) return fail(HB2_ERR_SIZE, "hb2_jacobi_ell: needs a square matrix");
+    // a Q1 grid operator: several sweeps a pass, in an even number of passes so that the
+    // result ends in x (one sweep: the plain pass below)
+    if (A->q1g_m && sweeps >= 2)
+    {
+        uint64_t passes = (sweeps + kQ1SweepMax - 1) / kQ1SweepMax;
+        passes += passes & 1;
+        void * from = x, * to = tmp;
+        for (; passes > 0; --passes)
+        {
+            Q1SweepPass p;
+            p.sweeps = (int)((sweeps + passes - 1) / passes);
+            sweeps -= p.sweeps;
+            p.pvec = true;
+            p.x = from;
+            p.b = b;
+            p.jac = P;
+            p.y = to;
+            const int st = launch_q1_sweep(A, p, stream);
+            if (st) return st;
+            std::swap(from, to);
+        }
+        return HB2_OK;
+    }
     // ping-pong: sweep s reads cur, writes nxt (true Jacobi, as the reference's
     // separate defect / element product / sum passes)
     void * cur = x, * nxt = tmp;

@@ -702,7 +702,7 @@ namespace hb2
         return autotune(A, stream);
     }
 
-    int ell_build_compact(hb2_ell_s * A, cudaStream_t stream)
+    static int build_layouts(hb2_ell_s * A, cudaStream_t stream)
     {
         // HB2_ELL_COMPACT=0 and matrices below kShapeMinRows: the plain layout in its
         // default (or pinned) shape, no timing; below kCompactMinRows, or without a
@@ -781,6 +781,15 @@ namespace hb2
             return HB2_OK;
         }
         return autotune(A, stream);
+    }
+
+    int ell_build_compact(hb2_ell_s * A, cudaStream_t stream)
+    {
+        const int st = build_layouts(A, stream);
+        if (st) return st;
+        // a pinned layout (HB2_ELL_COMPACT) runs everywhere, sweeps included
+        const char * pin = getenv("HB2_ELL_COMPACT");
+        return pin && *pin ? HB2_OK : ell_find_q1_grid(A, stream);
     }
 
     void ell_free_compact(hb2_ell_s * A)

@@ -133,6 +133,13 @@ struct hb2_ell_s
     // Their products run on kernels that know the rows' columns and weights
     // (launch_q1_transfer) instead of reading the matrix.
     int q1_transfer = 0;
+    // points per line when every row is one of the two rows of a Q1 grid operator
+    // (interior rows the nine values q1g_v, boundary rows the diagonal q1g_vb;
+    // checked row by row at creation, ell_find_q1_grid), 0 otherwise: several Jacobi
+    // sweeps and the transfers around them run as one pass (launch_q1_sweep)
+    uint32_t q1g_m = 0;
+    double q1g_v[9] = {};
+    double q1g_vb = 0;
 
     template <typename T> hb2::EllView<T> view() const
     {
@@ -305,6 +312,33 @@ namespace hb2
     // time the layouts and launch shapes the matrix admits, keep the fastest (ell_compact.cu)
     int ell_autotune(hb2_ell_s * A, cudaStream_t stream);
 
+    // Q1 sweep passes (q1_sweep.cu): `sweeps` (1 .. kQ1SweepMax) Jacobi sweeps of a matrix
+    // with q1g_m set, from x (+ the prolonged correction c) or from zero, into y != x;
+    // then (tail) nothing, the restriction of the new defect into coarse_b (coarse_zero
+    // cleared), or per-block partials of its squared norm in ws (*blocks of them).  jac:
+    // the Jacobi vector; without pvec it is omega / diag of the matrix, of which two
+    // entries are read.
+    constexpr int kQ1SweepMax = 4;
+    enum { kQ1TailNone = 0, kQ1TailRestrict = 1, kQ1TailNorm = 2 };
+    struct Q1SweepPass
+    {
+        int sweeps = 0;
+        bool zero_guess = false, pvec = false;
+        int tail = kQ1TailNone;
+        const void * x = nullptr, * c = nullptr, * b = nullptr, * jac = nullptr;
+        void * y = nullptr, * coarse_b = nullptr, * coarse_zero = nullptr;
+        const Workspace * ws = nullptr;
+        unsigned * blocks = nullptr;
+        // batched: vectors list[0 .. *count) of at most max_vec, vstride / cstride elements
+        // apart; the chunk height is chosen for nvec of them, at most cap blocks launched
+        const uint32_t * list = nullptr, * count = nullptr;
+        uint32_t nvec = 1, max_vec = 1;
+        uint64_t vstride = 0, cstride = 0, cap = 0;
+    };
+    bool q1_transfer_kernels_enabled();   // HB2_Q1_TRANSFER=0 turns them off (ell.cu)
+    int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream);
+    int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);
+
     // BLAS-1 helpers (blas1.cu) usable from other translation units.
     int launch_fill(int dt, void * x, double value, uint64_t n, cudaStream_t stream);
     int launch_copy(int dt, void * dst, const void * src, uint64_t n, cudaStream_t stream);
@@ -342,6 +376,10 @@ namespace hb2
         const void * jac;
     };
     constexpr uint64_t kSubMaxRows = 20000;
+    // levels that can run as sweep passes go into the cluster kernels only up to this many
+    // rows (a level-4 grid: whole level-6 solves 575 us with it there, 597 us without; the
+    // next larger grids are faster as sweep passes: 598 us with level 5 there, 668 with 5-6)
+    constexpr uint64_t kSubSweepRows = 300;
     int launch_subcycle(int dtype, const SubLevelDesc * lev, int top, int t1, int n_pre, int n_post, bool down,
                         cudaStream_t stream);
     int subcycle_prepare();

@@ -21,6 +21,7 @@
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -41,6 +42,7 @@ namespace hb2
         void * jac = 0;      // omega / diag(A)
         int keep = 0;        // kKeepL2 when the level's working set is near the L2 size
         bool rev_A = false, rev_R = false, rev_P = false;   // direction of the next pass
+        bool sweep = false;  // smoothing, defect and transfers in Q1 sweep passes (launch_q1_sweep)
 
         int pass(bool & rev)
         {
@@ -168,11 +170,74 @@ namespace hb2
         return st;
     }
 
-    // MGCycleCreation::_build_cycle (math/mg.hh:577-640); first_done: the level's
-    // first pre-smoothing sweep already ran (the fused loop)
-    static int record_cycle(hb2_mg_s * mg, uint32_t i, cudaStream_t s, bool first_done = false)
+    static int record_cycle(hb2_mg_s * mg, uint32_t i, cudaStream_t s, bool first_done = false, bool zero_guess = false,
+                            unsigned * norm_blocks = 0);
+
+    // `sweeps` Jacobi sweeps of level i in passes of at most kQ1SweepMax, the last one
+    // with `tail`; the iterate moves from `cur` to the level's other buffer and back
+    static int sweep_passes(hb2_mg_s * mg, uint32_t i, uint64_t sweeps, bool zero_guess, const void * c, int tail,
+                            void *& cur, unsigned * norm_blocks, cudaStream_t s)
     {
         MgLevel & L = mg->lev[i];
+        for (uint64_t passes = (sweeps + kQ1SweepMax - 1) / kQ1SweepMax; passes > 0; --passes)
+        {
+            Q1SweepPass p;
+            p.sweeps = (int)((sweeps + passes - 1) / passes);
+            sweeps -= p.sweeps;
+            p.zero_guess = zero_guess;
+            p.x = cur;
+            p.c = c;
+            p.b = L.b;
+            p.jac = L.jac;
+            p.y = cur == L.x ? L.tmp : L.x;
+            if (passes == 1)
+            {
+                p.tail = tail;
+                p.ws = mg->ws;
+                p.blocks = norm_blocks;
+                if (tail == kQ1TailRestrict)
+                {
+                    // a coarser level that starts its own sweep passes from zero reads no x
+                    p.coarse_b = mg->lev[i - 1].b;
+                    p.coarse_zero = mg->lev[i - 1].sweep && (int)i - 1 != mg->sub_top ? 0 : mg->lev[i - 1].x;
+                }
+            }
+            int st = launch_q1_sweep(L.A, p, s);
+            if (st) return st;
+            cur = p.y;
+            zero_guess = false;
+            c = 0;
+        }
+        return HB2_OK;
+    }
+
+    // the cycle of a level whose smoothing, defect and transfers run as sweep passes:
+    // one pass down (sweeps, defect, restriction), one up (prolongation, sweeps, on the
+    // finest level the norm's partials) while at most kQ1SweepMax sweeps are asked for
+    static int record_sweep_cycle(hb2_mg_s * mg, uint32_t i, cudaStream_t s, bool zero_guess, unsigned * norm_blocks)
+    {
+        MgLevel & L = mg->lev[i];
+        void * cur = L.x;
+        int st = sweep_passes(mg, i, mg->prm.n_pre_smooth, zero_guess, 0, kQ1TailRestrict, cur, 0, s);
+        if (! st) st = record_cycle(mg, i - 1, s, false, true);
+        if (! st && mg->prm.cycle == 1 && i - 1 != 0) st = record_cycle(mg, i - 1, s);
+        if (! st)
+            st = sweep_passes(mg, i, mg->prm.n_post_smooth, false, mg->lev[i - 1].x,
+                              norm_blocks ? kQ1TailNorm : kQ1TailNone, cur, norm_blocks, s);
+        if (! st && cur != L.x) st = launch_copy(mg->dtype, L.x, cur, L.n, s);
+        return st;
+    }
+
+    // MGCycleCreation::_build_cycle (math/mg.hh:577-640); first_done: the level's
+    // first pre-smoothing sweep already ran (the fused loop); zero_guess: the level
+    // starts from x = 0 (with sweep passes x itself need not hold zeros); norm_blocks
+    // (finest level with sweep passes): the number of partials of ||b - A x||^2 left in
+    // the workspace
+    static int record_cycle(hb2_mg_s * mg, uint32_t i, cudaStream_t s, bool first_done, bool zero_guess,
+                            unsigned * norm_blocks)
+    {
+        MgLevel & L = mg->lev[i];
+        if (L.sweep && ! first_done && (int)i > mg->sub_top) return record_sweep_cycle(mg, i, s, zero_guess, norm_blocks);
         if ((int)i == mg->sub_top) return record_small_levels(mg, s);
         if (i == 0) return coarse_solve(mg, s);
         MgLevel & C = mg->lev[i - 1];
@@ -186,6 +251,12 @@ namespace hb2
         if (! st) st = launch_ell(L.P, kAdd, C.x, L.x, 0, 0, 0, 0, 0, mg->ws, s, L.pass(L.rev_P));
         if (! st) st = smooth(mg, L, mg->prm.n_post_smooth, s);
         return st;
+    }
+
+    // the finest level's post-smoothing leaves the convergence norm's partials
+    static bool norm_in_sweep(const hb2_mg_s * mg)
+    {
+        return mg->lev[mg->nlev - 1].sweep && (int)mg->nlev - 1 > mg->sub_top && ! mg->fused_norm;
     }
 
     static int finest_norm(hb2_mg_s * mg, cudaStream_t s)
@@ -224,6 +295,59 @@ namespace hb2
         const double rc = *norm;
         const bool stop = rc < eps * *r0 || ! (rc == rc) || it >= max_iters;
         cudaGraphSetConditional(h, stop ? 0u : 1u);
+    }
+
+    // the same after a cycle that left the norm's partials (norm_in_sweep): their sum in
+    // the order of sum_partials_kernel, the root, the decision, in one launch
+    __global__ void __launch_bounds__(1024) mg_loop_decide_sum_kernel(const double * __restrict__ partials, unsigned G,
+                                                                      double * norm, const double * r0,
+                                                                      uint64_t * iters, uint64_t max_iters, double eps,
+                                                                      cudaGraphConditionalHandle h)
+    {
+        __shared__ double scratch[32];
+        pdl_entry();
+        double s = 0.0;
+        for (unsigned b = threadIdx.x; b < G; b += blockDim.x) s += partials[b];
+        s = block_sum(s, scratch);
+        if (threadIdx.x != 0) return;
+        const uint64_t it = *iters + 1;
+        *iters = it;
+        const double rc = sqrt(s);
+        *norm = rc;
+        const bool stop = rc < eps * *r0 || ! (rc == rc) || it >= max_iters;
+        cudaGraphSetConditional(h, stop ? 0u : 1u);
+    }
+
+    // one cycle and the convergence norm into norm_dev, without the decision
+    static int record_cycle_and_norm(hb2_mg_s * mg, cudaStream_t s)
+    {
+        unsigned G = 0;
+        const bool fused = norm_in_sweep(mg);
+        int st = record_cycle(mg, mg->nlev - 1, s, false, false, fused ? &G : 0);
+        if (st) return st;
+        if (! fused) return finest_norm(mg, s);
+        launch_sum_partials(mg->ws->partials, G, 1, mg->norm_dev, 1, s);
+        HB2_LAUNCH_CHECK("MG cycle: norm");
+        return HB2_OK;
+    }
+
+    // one cycle, its convergence norm and the loop's decision (the WHILE body)
+    static int record_cycle_and_decide(hb2_mg_s * mg, cudaStream_t s, cudaGraphConditionalHandle h)
+    {
+        unsigned G = 0;
+        const bool fused = norm_in_sweep(mg);
+        int st = record_cycle(mg, mg->nlev - 1, s, false, false, fused ? &G : 0);
+        if (! st && ! fused) st = finest_norm(mg, s);
+        if (st) return st;
+        if (fused)
+            launch_pdl(mg_loop_decide_sum_kernel, dim3(1), dim3(1024), 0, s, (const double *)mg->ws->partials, G,
+                       mg->norm_dev, (const double *)mg->r0_dev, mg->iters_dev, mg->prm.max_iters, mg->prm.eps_relative, h);
+        else
+            launch_pdl(mg_loop_decide_kernel, dim3(1), dim3(1), 0, s, mg->norm_dev, mg->r0_dev, mg->iters_dev,
+                       mg->prm.max_iters, mg->prm.eps_relative, h);
+        count_launches(1);
+        HB2_LAUNCH_CHECK("MG loop: decide kernel");
+        return HB2_OK;
     }
 
     // the fused loop's decision, after the first sweep of the cycle that would be
@@ -335,16 +459,7 @@ namespace hb2
         }
         else
         {
-            st = record_cycle(mg, mg->nlev - 1, mg->cap2);
-            if (! st) st = finest_norm(mg, mg->cap2);
-            if (! st)
-            {
-                launch_pdl(mg_loop_decide_kernel, dim3(1), dim3(1), 0, mg->cap2, mg->norm_dev, mg->r0_dev,
-                           mg->iters_dev, mg->prm.max_iters, mg->prm.eps_relative, h);
-                count_launches(1);
-                e = cudaGetLastError();
-                if (e != cudaSuccess) return capture_error(e, "decide kernel", mg);
-            }
+            st = record_cycle_and_decide(mg, mg->cap2, h);
             if (st) { capture_error(cudaSuccess, "", mg); return st; }
         }
         mg->body_kernels = hb2_launch_count() - body0;
@@ -368,8 +483,7 @@ namespace hb2
         HB2_CUDA(cudaStreamBeginCapture(mg->cap, cudaStreamCaptureModeThreadLocal));
         uint64_t before = hb2_launch_count();
         reset_directions(mg);
-        int st = record_cycle(mg, mg->nlev - 1, mg->cap);
-        if (! st) st = finest_norm(mg, mg->cap);
+        int st = record_cycle_and_norm(mg, mg->cap);
         if (! st)
         {
             cudaError_t e = cudaMemcpyAsync(mg->ws->host_scalars, mg->norm_dev, sizeof(double), cudaMemcpyDeviceToHost, mg->cap);
@@ -471,12 +585,22 @@ namespace hb2
         // measured slower on B200 than down / coarse CG / up as three)
         mg->sub_top = -1;
         mg->sub_t1 = 0;
+        mg->fused_norm = mg->nlev >= 2 && mg->prm.n_pre_smooth >= 1 && env_u64("HB2_MG_FUSED_NORM", 0) != 0;
+        for (uint32_t i = 1; i < mg->nlev; ++i)
+        {
+            MgLevel & L = mg->lev[i];
+            const int q = L.P->q1_transfer;
+            L.sweep = L.A->q1g_m && q > 0 && L.R->q1_transfer == -q && L.A->q1g_m == (1u << q) + 1 &&
+                      mg->prm.n_pre_smooth >= 1 && mg->prm.n_post_smooth >= 1 && q1_transfer_kernels_enabled() &&
+                      ! mg->fused_norm;
+        }
         const uint64_t max_rows = env_u64("HB2_SUB_MAX_ROWS", kSubMaxRows);
+        const uint64_t sweep_rows = std::min<uint64_t>(max_rows, kSubSweepRows);
         const uint64_t local_rows = env_u64("HB2_SUB_LOCAL_ROWS", kSubLocalRows);
         if (! mg->prm.no_fused_levels && mg->prm.cycle == 0 && mg->prm.n_pre_smooth < (1u << 20) &&
             mg->prm.n_post_smooth < (1u << 20))
             for (uint32_t i = 1; i < mg->nlev && i < 10; ++i)
-                if (mg->lev[i].n <= max_rows) mg->sub_top = (int)i;
+                if (mg->lev[i].n <= (mg->lev[i].sweep ? sweep_rows : max_rows)) mg->sub_top = (int)i;
         if (mg->sub_top >= 1)
         {
             for (int i = 1; i <= mg->sub_top; ++i)
@@ -498,8 +622,7 @@ namespace hb2
             HB2_CUDA(cudaStreamSynchronize(stream));
         }
         HB2_CUDA(cudaStreamSynchronize(stream));
-        mg->fused_norm = mg->nlev >= 2 && mg->sub_top < (int)mg->nlev - 1 && mg->prm.n_pre_smooth >= 1 &&
-                         env_u64("HB2_MG_FUSED_NORM", 0) != 0;
+        mg->fused_norm = mg->fused_norm && mg->sub_top < (int)mg->nlev - 1;
         mg->sub_fused = mg->sub_top >= 1 && env_u64("HB2_SUB_FUSED", 0) != 0 &&
                         subvcycle_supported(mg->lev[0].A, mg->coarse64);
         // prime the coarse kernel's shared-memory attribute outside the capture
@@ -782,14 +905,8 @@ namespace hb2
         }
         else
         {
-            st = record_cycle(mg, mg->nlev - 1, mg->cap3);
-            if (! st) st = finest_norm(mg, mg->cap3);
+            st = record_cycle_and_decide(mg, mg->cap3, hi);
             if (st) return ir_capture_error(cudaSuccess, "", mg, st);
-            launch_pdl(mg_loop_decide_kernel, dim3(1), dim3(1), 0, mg->cap3, mg->norm_dev, mg->r0_dev, mg->iters_dev,
-                       mg->prm.max_iters, mg->prm.eps_relative, hi);
-            count_launches(1);
-            e = cudaGetLastError();
-            if (e != cudaSuccess) return ir_capture_error(e, "IR inner decide", mg);
         }
         mg->ir_inner_body_kernels = hb2_launch_count() - ibody0;
         e = cudaStreamEndCapture(mg->cap3, &ibody);

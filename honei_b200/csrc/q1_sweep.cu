@@ -1,0 +1,124 @@
+// Which matrices the Q1 sweep kernel (q1_sweep.cuh) serves, and its launch.
+#include "q1_sweep_impl.cuh"
+
+
+namespace hb2
+{
+    int q1_sweep_f64(const Q1SweepArgs<double> & g, bool wide, bool uni, int S, int head, int tail, bool pvec,
+                     const SweepLaunch & l);
+    int q1_sweep_f32(const Q1SweepArgs<float> & g, bool wide, bool uni, int S, int head, int tail, bool pvec,
+                     const SweepLaunch & l);
+
+    // every row against the two rows of a Q1 grid operator: interior rows hold the nine
+    // couplings of v in ascending column order, boundary rows one diagonal entry vb in slot 0
+    template <typename T>
+    __global__ void q1_grid_check_kernel(EllView<T> A, uint32_t m, const T * __restrict__ ref, int * bad)
+    {
+        const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+        if (r >= A.rows) return;
+        const uint32_t i = (uint32_t)(r / m), j = (uint32_t)(r - (uint64_t)i * m);
+        const bool bnd = i == 0 || j == 0 || i == m - 1 || j == m - 1;
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+        {
+            const int32_t c = A.col[k * A.ld + r];
+            const T v = A.val[k * A.ld + r];
+            if (bnd) ok = ok && (k == 0 ? (c == (int32_t)r && v == ref[9]) : c < 0);
+            else ok = ok && c == (int32_t)((int64_t)r + (k / 3 - 1) * (int64_t)m + (k % 3 - 1)) && v == ref[k];
+        }
+        if (! ok) *bad = 1;
+    }
+
+    template <typename T>
+    static int find_grid_typed(hb2_ell_s * A, uint32_t m, cudaStream_t stream)
+    {
+        const EllView<T> V = A->view<T>();
+        T ref[10];
+        char * d = 0;
+        HB2_CUDA(cudaMalloc(&d, 10 * sizeof(T) + sizeof(int) + 8));
+        T * dref = (T *)d;
+        int * dbad = (int *)(d + 10 * sizeof(T));
+        cudaError_t e = cudaMemsetAsync(dbad, 0, sizeof(int), stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpy2DAsync(dref, sizeof(T), V.val + m + 1, V.ld * sizeof(T), sizeof(T), 9,
+                                  cudaMemcpyDeviceToDevice, stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(dref + 9, V.val, sizeof(T), cudaMemcpyDeviceToDevice, stream);
+        int bad = 1;
+        if (e == cudaSuccess)
+        {
+            q1_grid_check_kernel<T><<<ceil_div(A->rows, 256), 256, 0, stream>>>(V, m, dref, dbad);
+            count_launches(1);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(ref, dref, sizeof(ref), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        cudaFree(d);
+        if (e != cudaSuccess) return cuda_status(e, "Q1 grid check");
+        if (bad) return HB2_OK;
+        for (int k = 0; k < 9; ++k) A->q1g_v[k] = (double)ref[k];
+        A->q1g_vb = (double)ref[9];
+        A->q1g_m = m;
+        return HB2_OK;
+    }
+
+    int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream)
+    {
+        A->q1g_m = 0;
+        if (A->rows != A->cols || A->K != 9 || A->rows < 9 || A->rows >= (1ull << 31)) return HB2_OK;
+        uint64_t m = 3;
+        while (m * m < A->rows) ++m;
+        if (m * m != A->rows) return HB2_OK;
+        return A->dtype == HB2_F64 ? find_grid_typed<double>(A, (uint32_t)m, stream)
+                                   : find_grid_typed<float>(A, (uint32_t)m, stream);
+    }
+
+    template <typename T>
+    static int launch_typed(const hb2_ell_s * A, const Q1SweepPass & p, const SweepLaunch & l)
+    {
+        Q1SweepArgs<T> g = {};
+        bool uni = true;
+        for (int k = 0; k < 9; ++k)
+        {
+            g.v[k] = (T)A->q1g_v[k];
+            if (k != 4) uni = uni && A->q1g_v[k] == A->q1g_v[0];
+        }
+        g.vb = (T)A->q1g_vb;
+        g.m = (int)A->q1g_m;
+        g.mc = (g.m + 1) / 2;
+        g.x = (const T *)p.x;
+        g.c = (const T *)p.c;
+        g.b = (const T *)p.b;
+        g.jac = (const T *)p.jac;
+        g.y = (T *)p.y;
+        g.cb = (T *)p.coarse_b;
+        g.cz = (T *)p.coarse_zero;
+        g.partials = p.ws ? p.ws->partials : nullptr;
+        g.list = p.list;
+        g.count = p.count;
+        g.vs = p.vstride;
+        g.cs = p.cstride;
+        // FP64 columns a lane: two from level 9 (9.4 us a pass against 9.9 with one), one
+        // below (level 8: 6.7 us), where a strip of 20 owned columns leaves more warps
+        const bool wide = g.m >= 400;
+        if constexpr (sizeof(T) == 8)
+            return q1_sweep_f64(g, wide, uni, p.sweeps, p.zero_guess ? kSweepZero : kSweepLoad, p.tail, p.pvec, l);
+        else
+            return q1_sweep_f32(g, wide, uni, p.sweeps, p.zero_guess ? kSweepZero : kSweepLoad, p.tail, p.pvec, l);
+    }
+
+    int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream)
+    {
+        if (! A->q1g_m || p.sweeps < 1 || p.sweeps > kQ1SweepMax) return fail(HB2_ERR_UNSUPPORTED, "Q1 sweep");
+        SweepLaunch l;
+        l.nvec = p.list ? p.nvec : 1;
+        l.max_vec = p.list ? p.max_vec : 1;
+        l.cap = p.cap;
+        l.max_partials = p.ws ? p.ws->max_blocks : 0;
+        l.blocks = p.blocks;
+        l.stream = stream;
+        return A->dtype == HB2_F64 ? launch_typed<double>(A, p, l) : launch_typed<float>(A, p, l);
+    }
+}
