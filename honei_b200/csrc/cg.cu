@@ -240,7 +240,7 @@ namespace hb2
     {
         if (A->K == 0 || A->K > 9 || A->rows > 128) return false;
         const int rpl = (int)((A->rows + 31) / 32);
-        const size_t smem = 3 * A->rows * sizeof(T) + 16;
+        const size_t smem = (3 * A->rows + 1) * sizeof(T) + 16;
         EllView<T> v = A->view<T>();
         const S * bp = (const S *)b;
         S * xp = (S *)x;

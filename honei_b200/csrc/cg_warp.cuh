@@ -31,6 +31,24 @@ namespace hb2
         return fabs(d) > Eps<T>::v() ? d : Eps<T>::v();
     }
 
+    // The sum of v over the warp, in every lane, by two FP64 tensor-core products instead of
+    // five shuffle rounds: ones(8x4) * B(4x8) with lane l's value in B[l % 4][l / 4] sums
+    // groups of four lanes, each lane receives two neighbouring groups' sums and adds them,
+    // and S(8x4) * ones(4x8) sums those four values.  Measured (B200): 66 cycles against 176
+    // (a 64-bit shuffle and its add take 35, a product 29).  Every product is by one, so the
+    // result is a sum of the 32 values in a fixed order.
+    __device__ __forceinline__ double warp_sum_mma(double v)
+    {
+        double d0, d1, e0, e1;
+        const double one = 1.0, zero = 0.0;
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
+                     : "=d"(d0), "=d"(d1) : "d"(one), "d"(v), "d"(zero), "d"(zero));
+        const double s = d0 + d1;
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
+                     : "=d"(e0), "=d"(e1) : "d"(s), "d"(one), "d"(zero), "d"(zero));
+        return e0;
+    }
+
     // ------------------------------------------------------------------ one warp
     // Latency-bound coarse solves (the MG coarsest level has 81 unknowns and runs
     // a hundred iterations per V-cycle): one warp, no block barriers, reductions
@@ -71,7 +89,7 @@ namespace hb2
     // FP32 hierarchy can run its coarsest solve in FP64 on an FP64 copy of the
     // coarse operator: b is widened on load, x rounded on store).
     //
-    // cg_warp_reg runs in one full warp (lane = threadIdx.x & 31) and needs 3n
+    // cg_warp_reg runs in one full warp (lane = threadIdx.x & 31) and needs 3n + 1
     // elements of T in shared memory; it is called by cg_warp_reg_kernel and by
     // the fused small-level V-cycle kernel (subcycle.cu), which writes b earlier
     // in the same launch -- hence plain (coherent) loads of b, no __restrict__.
@@ -83,8 +101,12 @@ namespace hb2
         typedef Arith<T> M;
         constexpr int K = 9;
         const int n = (int)Ag.rows, lane = threadIdx.x & 31;
-        T * sp = smem;            // p (and x for the initial defect)
-        T * sa = sp + n;          // first dot operand (exact mode)
+        // p (and x for the initial defect), then a zero that empty slots gather; the tree
+        // modes alternate between two such vectors, so that one barrier an iteration orders
+        // the gathers of the old one before the writes of the new one
+        T * sp = smem;
+        T * sp2 = sp + n + 1;
+        T * sa = sp + n + 1;      // first dot operand (exact mode)
         T * sb = sa + n;          // second dot operand (exact mode)
         T av[RPL][K];
         int ac[RPL][K];
@@ -135,7 +157,23 @@ namespace hb2
 #pragma unroll
             for (int j = 0; j < RPL; ++j)
                 if (lane + 32 * j < n) s = fma((double)a[j], (double)bb[j], s);
-            return (T)warp_sum(s);
+            return (T)warp_sum_mma(s);
+        };
+        // the tree modes' product: three chains of three fused terms a row, no branches
+        auto spmv_tree = [&](T (&out)[RPL], const T * v) {
+#pragma unroll
+            for (int j = 0; j < RPL; ++j)
+            {
+                T s[3];
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                {
+                    s[q] = M::mul(av[j][3 * q], v[ac[j][3 * q] >= 0 ? ac[j][3 * q] : n]);
+                    s[q] = M::fma(av[j][3 * q + 1], v[ac[j][3 * q + 1] >= 0 ? ac[j][3 * q + 1] : n], s[q]);
+                    s[q] = M::fma(av[j][3 * q + 2], v[ac[j][3 * q + 2] >= 0 ? ac[j][3 * q + 2] : n], s[q]);
+                }
+                out[j] = M::add(M::add(s[0], s[1]), s[2]);
+            }
         };
         T tmp[RPL];
         spmv(tmp);
@@ -164,14 +202,16 @@ namespace hb2
             //   x += a p; r -= a s; w = A r; g = (r, r); d = (w, r);
             //   b = g / g_old; a = g / (d - b g / a_old); p = r + b p; s = w + b s
             T sr[RPL], wr[RPL];
-            spmv(wr);   // w0 = A r0 (sp holds r0 = p0)
+            if (lane == 0) sp[n] = sp2[n] = T(0);
+            __syncwarp();
+            spmv_tree(wr, sp);   // w0 = A r0 (sp holds r0 = p0)
             T gam = alpha, del;
             {
                 double s1 = 0.0;
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
                     if (lane + 32 * j < n) s1 = fma((double)wr[j], (double)rr[j], s1);
-                del = (T)warp_sum(s1);
+                del = (T)warp_sum_mma(s1);
             }
             T a = M::div(gam, guard(del));
             T inv_a = Recip<T>::rn(guard(a)), inv_g = Recip<T>::rn(guard(gam));
@@ -179,37 +219,31 @@ namespace hb2
             const T thr = M::mul(eps, initial), thr2 = M::mul(thr, thr), eps2 = M::mul(eps, eps);
 #pragma unroll
             for (int j = 0; j < RPL; ++j) sr[j] = wr[j];
+            T * cur = sp, * nxt = sp2;
             while (it < max_iters)
             {
-                const T ma = -a;
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
                 {
-                    xr[j] = M::add(xr[j], M::mul(a, pr[j]));
-                    rr[j] = M::add(rr[j], M::mul(ma, sr[j]));
+                    rr[j] = M::fma(-a, sr[j], rr[j]);
+                    if (lane + 32 * j < n) nxt[lane + 32 * j] = rr[j];
                 }
-                __syncwarp();   // every lane is done gathering the old r
-#pragma unroll
-                for (int j = 0; j < RPL; ++j)
-                    if (lane + 32 * j < n) sp[lane + 32 * j] = rr[j];
                 __syncwarp();
-                spmv(wr);
+#pragma unroll
+                for (int j = 0; j < RPL; ++j) xr[j] = M::fma(a, pr[j], xr[j]);
+                spmv_tree(wr, nxt);
+                T * t = cur;
+                cur = nxt;
+                nxt = t;
                 double s1 = 0.0, s2 = 0.0;
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
-                    if (lane + 32 * j < n)
-                    {
-                        s1 = fma((double)rr[j], (double)rr[j], s1);
-                        s2 = fma((double)wr[j], (double)rr[j], s2);
-                    }
+                    if (lane + 32 * j < n) s1 = fma((double)rr[j], (double)rr[j], s1);
+                const T g = (T)warp_sum_mma(s1);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                {
-                    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-                    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-                }
-                const T g = (T)s1;
-                del = (T)s2;
+                for (int j = 0; j < RPL; ++j)
+                    if (lane + 32 * j < n) s2 = fma((double)wr[j], (double)rr[j], s2);
+                del = (T)warp_sum_mma(s2);
                 ++it;
                 if (g < thr2 || g < eps2 || it == max_iters)
                 {
@@ -218,18 +252,17 @@ namespace hb2
                     break;
                 }
                 // single-rounded reciprocals instead of IEEE divisions (this mode is
-                // not the reference's order anyway)
-                const T b = M::mul(g, inv_g);
-                a = M::mul(g, Recip<T>::rn(guard(M::sub(del, M::mul(M::mul(b, g), inv_a)))));
+                // not the reference's order anyway); 1/g and b do not wait for (w, r)
+                const T b = M::mul(g, inv_g), bg = M::mul(M::mul(b, g), inv_a);
+                inv_g = Recip<T>::rn(guard(g));
+                a = M::mul(g, Recip<T>::rn(guard(M::sub(del, bg))));
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
                 {
-                    pr[j] = M::add(rr[j], M::mul(b, pr[j]));
-                    sr[j] = M::add(wr[j], M::mul(b, sr[j]));
+                    pr[j] = M::fma(b, pr[j], rr[j]);
+                    sr[j] = M::fma(b, sr[j], wr[j]);
                 }
                 inv_a = Recip<T>::rn(guard(a));
-                inv_g = Recip<T>::rn(guard(g));
-                gam = g;
             }
             it = max_iters;   // done: skip the loop below
         }

@@ -349,7 +349,7 @@ namespace hb2
     __global__ void __launch_bounds__(kSubVThreads, 1) mg_sub_vcycle_kernel(const __grid_constant__ SubVCycle<T> sc)
     {
         pdl_entry();
-        __shared__ double cg_smem[3 * 96];
+        __shared__ double cg_smem[3 * 96 + 1];
         cg::cluster_group cluster = cg::this_cluster();
         const Team<false, PL> all = {cluster.block_rank() * blockDim.x + threadIdx.x, cluster.num_blocks() * blockDim.x};
         const SubPat<T> none = {nullptr, nullptr};
