@@ -339,6 +339,28 @@ namespace hb2
     int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream);
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);
 
+    // the bottom of a V-cycle, levels 0 (coarsest, CG) .. top, in one block (q1_bottom.cu):
+    // A[1 .. top] Q1 grid operators of at most 33 points per line that q1_bottom_fits
+    // accepts, each twice as fine as the one before, A[0] at most 96 rows; from zero or from x
+    constexpr int kQ1BottomLevels = 4;
+    struct Q1Bottom
+    {
+        const hb2_ell_s * A[kQ1BottomLevels + 1] = {};
+        const void * jac[kQ1BottomLevels + 1] = {};
+        const hb2_ell_s * coarse64 = nullptr;
+        int top = 0, n_pre = 0, n_post = 0, exact = 0;
+        bool zero_guess = false;
+        const void * b = nullptr;
+        void * x = nullptr;
+        uint64_t max_iters = 0;
+        double eps = 0;
+        uint64_t * used = nullptr;
+        double * defect = nullptr;
+    };
+    bool q1_bottom_fits(const hb2_ell_s * A);
+    bool q1_bottom_coarse_fits(const hb2_ell_s * C);
+    int launch_q1_bottom(int dtype, const Q1Bottom & p, cudaStream_t s);
+
     // BLAS-1 helpers (blas1.cu) usable from other translation units.
     int launch_fill(int dt, void * x, double value, uint64_t n, cudaStream_t stream);
     int launch_copy(int dt, void * dst, const void * src, uint64_t n, cudaStream_t stream);

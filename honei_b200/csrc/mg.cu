@@ -79,6 +79,7 @@ struct hb2_mg_s
     int sub_top;             // levels 1..sub_top run as cluster kernels (-1: none)
     int sub_t1;              // of those, levels 1..sub_t1 run in one CTA
     bool sub_fused;          // levels 0..sub_top, coarse CG included, in one launch
+    int bottom_top;          // levels 0..bottom_top of a Q1 hierarchy run in one block (q1_bottom.cu); -1: none
     hb2_ell_s * coarse64;    // FP64 copy of the coarsest operator (F32 hierarchies with coarse_fp64)
     double * ir_r;           // outer FP64 defect of hb2_ir_solve (allocated on first use, kept)
     // hb2_ir_solve as one CUDA graph, built for the outer operator and vectors of
@@ -173,6 +174,35 @@ namespace hb2
     static int record_cycle(hb2_mg_s * mg, uint32_t i, cudaStream_t s, bool first_done = false, bool zero_guess = false,
                             unsigned * norm_blocks = 0);
 
+    // level i of a V-cycle as its own sweep passes (not part of a fused bottom)
+    static bool in_sweeps(const hb2_mg_s * mg, uint32_t i)
+    {
+        return mg->lev[i].sweep && (int)i > mg->sub_top && (int)i > mg->bottom_top;
+    }
+
+    static int record_bottom(hb2_mg_s * mg, cudaStream_t s, bool zero_guess)
+    {
+        Q1Bottom p;
+        for (int i = 0; i <= mg->bottom_top; ++i)
+        {
+            p.A[i] = mg->lev[i].A;
+            p.jac[i] = mg->lev[i].jac;
+        }
+        p.coarse64 = mg->coarse64;
+        p.top = mg->bottom_top;
+        p.n_pre = (int)mg->prm.n_pre_smooth;
+        p.n_post = (int)mg->prm.n_post_smooth;
+        p.exact = mg->prm.coarse_exact;
+        p.zero_guess = zero_guess;
+        p.b = mg->lev[p.top].b;
+        p.x = mg->lev[p.top].x;
+        p.max_iters = mg->prm.max_iters_coarse;
+        p.eps = mg->prm.coarse_eps;
+        p.used = mg->coarse_used_dev;
+        p.defect = mg->coarse_def_dev;
+        return launch_q1_bottom(mg->dtype, p, s);
+    }
+
     // `sweeps` Jacobi sweeps of level i in passes of at most kQ1SweepMax, the last one
     // with `tail`; the iterate moves from `cur` to the level's other buffer and back
     static int sweep_passes(hb2_mg_s * mg, uint32_t i, uint64_t sweeps, bool zero_guess, const void * c, int tail,
@@ -197,9 +227,9 @@ namespace hb2
                 p.blocks = norm_blocks;
                 if (tail == kQ1TailRestrict)
                 {
-                    // a coarser level that starts its own sweep passes from zero reads no x
+                    // sweep passes and the fused bottom start from zero without reading x
                     p.coarse_b = mg->lev[i - 1].b;
-                    p.coarse_zero = mg->lev[i - 1].sweep && (int)i - 1 != mg->sub_top ? 0 : mg->lev[i - 1].x;
+                    p.coarse_zero = in_sweeps(mg, i - 1) || (int)i - 1 == mg->bottom_top ? 0 : mg->lev[i - 1].x;
                 }
             }
             int st = launch_q1_sweep(L.A, p, s);
@@ -237,7 +267,8 @@ namespace hb2
                             unsigned * norm_blocks)
     {
         MgLevel & L = mg->lev[i];
-        if (L.sweep && ! first_done && (int)i > mg->sub_top) return record_sweep_cycle(mg, i, s, zero_guess, norm_blocks);
+        if ((int)i == mg->bottom_top && ! first_done) return record_bottom(mg, s, zero_guess);
+        if (in_sweeps(mg, i) && ! first_done) return record_sweep_cycle(mg, i, s, zero_guess, norm_blocks);
         if ((int)i == mg->sub_top) return record_small_levels(mg, s);
         if (i == 0) return coarse_solve(mg, s);
         MgLevel & C = mg->lev[i - 1];
@@ -256,7 +287,7 @@ namespace hb2
     // the finest level's post-smoothing leaves the convergence norm's partials
     static bool norm_in_sweep(const hb2_mg_s * mg)
     {
-        return mg->lev[mg->nlev - 1].sweep && (int)mg->nlev - 1 > mg->sub_top && ! mg->fused_norm;
+        return in_sweeps(mg, mg->nlev - 1) && ! mg->fused_norm;
     }
 
     static int finest_norm(hb2_mg_s * mg, cudaStream_t s)
@@ -594,7 +625,16 @@ namespace hb2
                       mg->prm.n_pre_smooth >= 1 && mg->prm.n_post_smooth >= 1 && q1_transfer_kernels_enabled() &&
                       ! mg->fused_norm;
         }
-        const uint64_t max_rows = env_u64("HB2_SUB_MAX_ROWS", kSubMaxRows);
+        // a Q1 hierarchy's smallest levels and its coarse CG in one block (V-cycles)
+        mg->bottom_top = -1;
+        if (! mg->prm.no_fused_levels && mg->prm.cycle == 0 && q1_bottom_coarse_fits(mg->lev[0].A) &&
+            mg->prm.n_pre_smooth < (1u << 20) && mg->prm.n_post_smooth < (1u << 20))
+            for (uint32_t i = 1; i < mg->nlev && (int)i <= kQ1BottomLevels; ++i)
+            {
+                if (! mg->lev[i].sweep || ! q1_bottom_fits(mg->lev[i].A)) break;
+                mg->bottom_top = (int)i;
+            }
+        const uint64_t max_rows = mg->bottom_top >= 1 ? 0 : env_u64("HB2_SUB_MAX_ROWS", kSubMaxRows);
         const uint64_t sweep_rows = std::min<uint64_t>(max_rows, kSubSweepRows);
         const uint64_t local_rows = env_u64("HB2_SUB_LOCAL_ROWS", kSubLocalRows);
         if (! mg->prm.no_fused_levels && mg->prm.cycle == 0 && mg->prm.n_pre_smooth < (1u << 20) &&
