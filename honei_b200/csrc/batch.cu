@@ -54,7 +54,10 @@ namespace hb2
 
     constexpr int kMaxGroups = 14;
     constexpr int kOuterThreads = 256;
-    constexpr int kOuterRows = 2;   // rows per thread: one 128-bit load of FP64 values per slot
+    // rows per thread and work item, interleaved over the block.  Four instead of two halves
+    // the reductions (a block sum, a fence and two tickets an item); measured with the stencil
+    // product below on the 128-system batch, see hb2_batch_s.
+    constexpr int kOuterRows = 4;
 
     constexpr int kMaxLevels = 16;
 
@@ -95,6 +98,9 @@ namespace hb2
     struct OuterGroup
     {
         EllView<double> A;            // FP64 operator of the finest level (plain layout)
+        uint32_t m;                   // points per line when it is a Q1 grid operator (q1g_m), else 0
+        double a[9], ab;              // its interior row and boundary diagonal
+        int clear32;                  // the first sweep of the level reads the inner correction: clear it
         uint64_t n, vs;               // rows, stride of the FP64 vectors
         uint64_t vs32;                // stride of the level's FP32 vectors
         uint32_t first, count;        // vector range
@@ -119,42 +125,35 @@ namespace hb2
         return fabs(d) > DBL_EPSILON ? d : __dmul_rn(DBL_EPSILON, __ddiv_rn(d, fabs(d)));
     }
 
-    // acc[i] = sum_k A(r0 + i, k) * x(col), slot order, separately rounded
-    // (la/product.hh:148-206)
-    template <int KT>
-    __device__ __forceinline__ void rows_product(const EllView<double> & A, uint64_t r0, const double * x,
-                                                 double (&acc)[kOuterRows])
+    // sum_k A(row, k) * x(col), slot order, separately rounded (la/product.hh:148-206); from
+    // the grid when the operator is a Q1 one -- the matrix is 108 bytes a row against the 8
+    // of x, and every vector of the level would stream it again
+    __device__ __forceinline__ double row_product(const OuterGroup & G, uint64_t row, const double * x)
     {
-        acc[0] = acc[1] = 0.0;
-        if (r0 >= A.rows) return;
-        const int K = KT > 0 ? KT : (int)A.K;
-        if constexpr (KT > 0)
+        double acc = 0.0;
+        if (G.m)
         {
-            double2 v[KT];
-            int2 c[KT];
+            const uint32_t m = G.m, r = (uint32_t)row, i = r / m, j = r - i * m;
+            if (i == 0 || j == 0 || i == m - 1 || j == m - 1) return __dadd_rn(0.0, __dmul_rn(G.ab, __ldg(x + row)));
+            const double * c = x + row;
+            double xv[9];
 #pragma unroll
-            for (int k = 0; k < KT; ++k)
+            for (int q = 0; q < 3; ++q)
             {
-                v[k] = __ldg((const double2 *)(A.val + (uint64_t)k * A.ld + r0));
-                c[k] = __ldg((const int2 *)(A.col + (uint64_t)k * A.ld + r0));
+                xv[q] = __ldg(c - (int)m + (q - 1));
+                xv[3 + q] = __ldg(c + (q - 1));
+                xv[6 + q] = __ldg(c + (int)m + (q - 1));
             }
 #pragma unroll
-            for (int k = 0; k < KT; ++k)
-            {
-                if (c[k].x >= 0) acc[0] = __dadd_rn(acc[0], __dmul_rn(v[k].x, __ldg(x + c[k].x)));
-                if (c[k].y >= 0) acc[1] = __dadd_rn(acc[1], __dmul_rn(v[k].y, __ldg(x + c[k].y)));
-            }
+            for (int q = 0; q < 9; ++q) acc = __dadd_rn(acc, __dmul_rn(G.a[q], xv[q]));
+            return acc;
         }
-        else
+        for (uint32_t k = 0; k < G.A.K; ++k)
         {
-            for (int k = 0; k < K; ++k)
-            {
-                const double2 vv = __ldg((const double2 *)(A.val + (uint64_t)k * A.ld + r0));
-                const int2 cc = __ldg((const int2 *)(A.col + (uint64_t)k * A.ld + r0));
-                if (cc.x >= 0) acc[0] = __dadd_rn(acc[0], __dmul_rn(vv.x, __ldg(x + cc.x)));
-                if (cc.y >= 0) acc[1] = __dadd_rn(acc[1], __dmul_rn(vv.y, __ldg(x + cc.y)));
-            }
+            const int32_t c = __ldg(G.A.col + (uint64_t)k * G.A.ld + row);
+            if (c >= 0) acc = __dadd_rn(acc, __dmul_rn(__ldg(G.A.val + (uint64_t)k * G.A.ld + row), __ldg(x + c)));
         }
+        return acc;
     }
 
     template <typename F>
@@ -195,33 +194,31 @@ namespace hb2
     // Phase A.  kNew: r = b - A x (math/cg.hh:161), ||r||^2; kRun: v = A p,
     // v.p (cg.hh:174-175).  Either way the inner rhs of the finest level gets
     // (float) r and the inner correction 0, ready for the preconditioner.
-    template <int KT>
     __global__ void __launch_bounds__(kOuterThreads) bpcg_phase_a_kernel(const __grid_constant__ OuterPlan P, SlotScalars S)
     {
         walk(P, S.live, S.plan->live_start, S.plan->live_item0, [&](const OuterGroup & G, uint32_t j, uint32_t lj, uint32_t blk) {
             const bool init = S.state[j] == kNew;
             const uint64_t o = (uint64_t)lj * G.vs, o32 = (uint64_t)j * G.vs32;
-            const uint64_t r0 = ((uint64_t)blk * kOuterThreads + threadIdx.x) * kOuterRows;
-            double acc[kOuterRows];
-            rows_product<KT>(G.A, r0, (init ? G.x : G.p) + o, acc);
+            const double * xp = (init ? G.x : G.p) + o;
             double part = 0.0;
 #pragma unroll
             for (int i = 0; i < kOuterRows; ++i)
             {
-                const uint64_t row = r0 + i;
+                const uint64_t row = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
                 if (row >= G.n) break;
+                const double acc = row_product(G, row, xp);
                 if (init)
                 {
-                    const double d = __dsub_rn(G.b[o + row], acc[i]);
+                    const double d = __dsub_rn(G.b[o + row], acc);
                     G.r[o + row] = d;
                     G.b32[o32 + row] = __double2float_rn(d);
-                    G.x32[o32 + row] = 0.f;
+                    if (G.clear32) G.x32[o32 + row] = 0.f;
                     part = fma(d, d, part);
                 }
                 else
                 {
-                    G.v[o + row] = acc[i];
-                    part = fma(acc[i], G.p[o + row], part);
+                    G.v[o + row] = acc;
+                    part = fma(acc, xp[row], part);
                 }
             }
             finish(G, lj, blk, part, S.red_a + j, [] {});
@@ -237,18 +234,17 @@ namespace hb2
             const double lambda = __ddiv_rn(S.an[j], guard_signed(S.red_a[j]));
             const double mlambda = -lambda;
             const uint64_t o = (uint64_t)lj * G.vs, o32 = (uint64_t)j * G.vs32;
-            const uint64_t r0 = ((uint64_t)blk * kOuterThreads + threadIdx.x) * kOuterRows;
             double part = 0.0;
 #pragma unroll
             for (int i = 0; i < kOuterRows; ++i)
             {
-                const uint64_t row = r0 + i;
+                const uint64_t row = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
                 if (row >= G.n) break;
                 G.x[o + row] = __dadd_rn(G.x[o + row], __dmul_rn(lambda, G.p[o + row]));
                 const double rr = __dadd_rn(G.r[o + row], __dmul_rn(mlambda, G.v[o + row]));
                 G.r[o + row] = rr;
                 G.b32[o32 + row] = __double2float_rn(rr);
-                G.x32[o32 + row] = 0.f;
+                if (G.clear32) G.x32[o32 + row] = 0.f;
                 part = fma(rr, rr, part);
             }
             finish(G, lj, blk, part, S.red_u + j, [] {});
@@ -391,12 +387,11 @@ namespace hb2
     {
         walk(P, S.plist, S.plan->prec_start, S.plan->prec_item0, [&](const OuterGroup & G, uint32_t j, uint32_t lj, uint32_t blk) {
             const uint64_t o = (uint64_t)lj * G.vs, o32 = (uint64_t)j * G.vs32;
-            const uint64_t r0 = ((uint64_t)blk * kOuterThreads + threadIdx.x) * kOuterRows;
             double part = 0.0;
 #pragma unroll
             for (int i = 0; i < kOuterRows; ++i)
             {
-                const uint64_t row = r0 + i;
+                const uint64_t row = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
                 if (row >= G.n) break;
                 part = fma(G.r[o + row], (double)G.x32[o32 + row], part);
             }
@@ -416,11 +411,10 @@ namespace hb2
             const bool fresh = S.fresh[j] != 0;
             const double t = S.tco[j];
             const uint64_t o = (uint64_t)lj * G.vs, o32 = (uint64_t)j * G.vs32;
-            const uint64_t r0 = ((uint64_t)blk * kOuterThreads + threadIdx.x) * kOuterRows;
 #pragma unroll
             for (int i = 0; i < kOuterRows; ++i)
             {
-                const uint64_t row = r0 + i;
+                const uint64_t row = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
                 if (row >= G.n) break;
                 const double z = (double)G.x32[o32 + row];
                 G.p[o + row] = fresh ? z : __dadd_rn(__dmul_rn(G.p[o + row], t), z);
@@ -461,6 +455,8 @@ namespace hb2
         uint64_t n = 0, vs = 0;
         uint32_t nv = 0;                 // vectors with a copy on this level (a prefix)
         float * x = 0, * b = 0, * store = 0, * tmp = 0, * jac = 0;
+        float * at = 0;                  // where the iterate is between the two legs (sweep passes)
+        bool sweep = false;              // smoothing, defect and transfers in Q1 sweep passes
     };
 
     struct BGroup
@@ -486,7 +482,6 @@ struct hb2_batch_s
     hb2_ell coarse64 = 0;
     hb2::OuterPlan plan;
     uint64_t outer_items = 0;           // largest number of outer work items of a step
-    bool outer_k9 = true;
     hb2::SlotScalars S;
     void * block = 0;                   // every device array of the batch
     uint64_t bytes = 0;
@@ -518,8 +513,7 @@ namespace hb2
         switch (which)
         {
             case 0:
-                if (B->outer_k9) launch_pdl(bpcg_phase_a_kernel<9>, grid, dim3(kOuterThreads), 0, s, B->plan, B->S);
-                else launch_pdl(bpcg_phase_a_kernel<0>, grid, dim3(kOuterThreads), 0, s, B->plan, B->S);
+                launch_pdl(bpcg_phase_a_kernel, grid, dim3(kOuterThreads), 0, s, B->plan, B->S);
                 break;
             case 1: launch_pdl(bpcg_update_kernel, grid, dim3(kOuterThreads), 0, s, B->plan, B->S); break;
             case 2: launch_pdl(bpcg_dot_z_kernel, grid, dim3(kOuterThreads), 0, s, B->plan, B->S); break;
@@ -549,6 +543,46 @@ namespace hb2
         return HB2_OK;
     }
 
+    // `sweeps` Jacobi sweeps of level i for every listed vector in passes of at most
+    // kQ1SweepMax; down: from zero, the last pass restricting the defect; up: the first
+    // pass adds the prolonged coarser correction
+    static int b_sweep_passes(hb2_batch_s * B, int i, uint64_t sweeps, bool down, float *& cur, cudaStream_t s)
+    {
+        BLevel & L = B->lev[i], & C = B->lev[i - 1];
+        bool first = true;
+        for (uint64_t passes = (sweeps + kQ1SweepMax - 1) / kQ1SweepMax; passes > 0; --passes)
+        {
+            Q1SweepPass p;
+            p.sweeps = (int)((sweeps + passes - 1) / passes);
+            sweeps -= p.sweeps;
+            p.zero_guess = down && first;
+            p.x = cur;
+            p.c = ! down && first ? C.x : nullptr;
+            p.b = L.b;
+            p.jac = L.jac;
+            p.y = cur == L.x ? L.tmp : L.x;
+            if (down && passes == 1)
+            {
+                p.tail = kQ1TailRestrict;
+                p.coarse_b = C.b;
+                p.coarse_zero = C.sweep ? nullptr : C.x;
+            }
+            p.list = B->S.plist;
+            p.count = &B->S.plan->vcount[i];
+            p.vstride = L.vs;
+            p.cstride = C.vs;
+            p.cap = B->grid_cap ? B->grid_cap : list_grid_cap();
+            // the vectors the chunk height is chosen for: all, or what the light step serves
+            p.nvec = B->grid_cap ? (uint32_t)std::min<uint64_t>(L.nv, B->light_rows / L.n + 1) : L.nv;
+            p.max_vec = L.nv;
+            const int st = launch_q1_sweep(L.A, p, s);
+            if (st) return st;
+            cur = (float *)p.y;
+            first = false;
+        }
+        return HB2_OK;
+    }
+
     // z = M r: one V-cycle over every vector the mask selects (MGCycleCreation
     // V::STATIC order, math/mg.hh:577-640), level by level
     static int b_vcycle(hb2_batch_s * B, cudaStream_t s)
@@ -558,6 +592,13 @@ namespace hb2
         {
             BLevel & L = B->lev[i], & C = B->lev[i - 1];
             if (L.nv == 0) continue;
+            if (L.sweep)
+            {
+                L.at = L.x;
+                const int st = b_sweep_passes(B, i, B->prm.n_pre_smooth, true, L.at, s);
+                if (st) return st;
+                continue;
+            }
             int st = b_smooth(B, L, B->prm.n_pre_smooth, s);
             Batch bt;
             bt.nvec = L.nv;
@@ -581,6 +622,13 @@ namespace hb2
         {
             BLevel & L = B->lev[i], & C = B->lev[i - 1];
             if (L.nv == 0) continue;
+            if (L.sweep)
+            {
+                st = b_sweep_passes(B, i, B->prm.n_post_smooth, false, L.at, s);
+                if (! st && L.at != L.x) st = launch_copy(HB2_F32, L.x, L.at, (uint64_t)L.nv * L.vs, s);
+                if (st) return st;
+                continue;
+            }
             Batch bp;
             bp.nvec = L.nv;
             bp.vstride = L.vs;
@@ -805,6 +853,15 @@ namespace hb2
         for (BGroup & g : B->grp)
             if (! st) st = hb2_ell_create_q1(&g.A64, HB2_F64, g.level, 1.0, stream);
         if (st) return st;
+        for (size_t i = 1; i < B->lev.size(); ++i)
+        {
+            BLevel & L = B->lev[i];
+            L.sweep = L.A->q1g_m && L.P->q1_transfer > 0 && L.A->q1g_m == (1u << L.P->q1_transfer) + 1 &&
+                      B->prm.n_pre_smooth >= 1 && B->prm.n_post_smooth >= 1 && q1_transfer_kernels_enabled();
+        }
+        // the light graph (2 blocks per SM) serves up to about two row blocks of
+        // work per block: ~150k live rows (a few systems of level 8 and below)
+        B->light_rows = (uint64_t)num_sms() * 2 * kEllThreads * 2;
         if (! cg_mixed_supported(B->coarse64))
             return fail(HB2_ERR_UNSUPPORTED, "hb2_batch_create_q1: the coarsest level needs <= 128 rows (level <= 3)");
         // one device block: level vectors | group vectors | reduction scratch | scalars
@@ -867,7 +924,6 @@ namespace hb2
         memset(&B->plan, 0, sizeof(B->plan));
         B->plan.ngroups = (int)B->grp.size();
         uint64_t blocks = 0;
-        B->outer_k9 = true;
         for (size_t i = 0; i < B->grp.size(); ++i)
         {
             BGroup & g = B->grp[i];
@@ -878,11 +934,14 @@ namespace hb2
             g.v = (double *)(base + go[i * 8 + 4]);
             OuterGroup & o = B->plan.g[i];
             o.A = g.A64->view<double>();
-            if (g.A64->K != 9) B->outer_k9 = false;
+            o.m = g.A64->q1g_m;
+            for (int k = 0; k < 9; ++k) o.a[k] = g.A64->q1g_v[k];
+            o.ab = g.A64->q1g_vb;
             o.n = g.n;
             o.vs = g.vs;
             const BLevel & L = B->lev[g.level - c];
             o.vs32 = L.vs;
+            o.clear32 = ! L.sweep;
             o.b32 = L.b;
             o.x32 = L.x;
             o.first = g.first;
@@ -917,9 +976,6 @@ namespace hb2
         HB2_CUDA(cudaStreamCreateWithFlags(&B->cap2, cudaStreamNonBlocking));
         st = build_step_graph(B, 0, &B->step_graph, &B->step_exec);
         if (! st) st = build_step_graph(B, (uint64_t)num_sms() * 2, &B->light_graph, &B->light_exec);
-        // the light graph (2 blocks per SM) serves up to about two row blocks of
-        // work per block: ~150k live rows (a few systems of level 8 and below)
-        B->light_rows = (uint64_t)num_sms() * 2 * kEllThreads * 2;
         B->vec_rows.assign(B->nvec, 0);
         for (uint32_t s = 0; s < B->nsys; ++s)
             for (uint32_t k = 0; k < B->sys_nrhs[s]; ++k) B->vec_rows[B->sys_first[s] + k] = q1_rows(B->sys_level[s]);
