@@ -333,6 +333,11 @@ namespace hb2
             if (red) HB2_CUDA(cudaMemsetAsync(red, 0, sizeof(double), stream));
             return HB2_OK;
         }
+        if (b.nvec == 1 && ! b.list && ! b.active && q1_single_applies(A, mode))
+        {
+            if (red && ! ws) return fail(HB2_ERR_ARG, "fused reduction without a workspace");
+            return launch_q1_single(A, mode, x, y, aux, red, want_sqrt, ws, stream);
+        }
         // the launch shape: the class's tuned one, except where a Q1 gather layout
         // hands this launch to the general row-pattern kernel (256 threads)
         const int cls = red != 0;

@@ -745,6 +745,8 @@ namespace hb2
     int launch_ir_defect(const hb2_ell_s * A, const double * x, const double * b, float * b32, float * x32,
                          double * r64, double * red, const Workspace * ws, cudaStream_t stream)
     {
+        if (A->dtype == HB2_F64 && q1_single_applies(A, kDefect))
+            return launch_q1_ir_defect(A, x, b, b32, x32, red, ws, stream);
         const uint64_t n = A->rows;
         const unsigned grid = ceil_div(n, kEllThreads);
         if (A->dtype == HB2_F64 && A->q1_full >= 0 && A->pat && A->pat_win_m && A->K == 9 && n > 0 &&

@@ -329,6 +329,7 @@ namespace hb2
         void * y = nullptr, * coarse_b = nullptr, * coarse_zero = nullptr;
         const Workspace * ws = nullptr;
         unsigned * blocks = nullptr;
+        float * y32 = nullptr, * z32 = nullptr;   // the refinement's defect (q1_sweep.cuh)
         // batched: vectors list[0 .. *count) of at most max_vec, vstride / cstride elements
         // apart; the chunk height is chosen for nvec of them, at most cap blocks launched
         const uint32_t * list = nullptr, * count = nullptr;
@@ -338,6 +339,13 @@ namespace hb2
     bool q1_transfer_kernels_enabled();   // HB2_Q1_TRANSFER=0 turns them off (ell.cu)
     int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream);
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);
+    // one product, defect or product with dot (kPlain, kDefect, kDot) as a streaming pass; the
+    // refinement's outer defect (kDefectIR)
+    bool q1_single_applies(const hb2_ell_s * A, int mode);
+    int launch_q1_single(const hb2_ell_s * A, int mode, const void * x, void * y, const void * b, double * red,
+                         int want_sqrt, const Workspace * ws, cudaStream_t stream);
+    int launch_q1_ir_defect(const hb2_ell_s * A, const double * x, const double * b, float * b32, float * x32,
+                            double * red, const Workspace * ws, cudaStream_t stream);
 
     // the bottom of a V-cycle, levels 0 (coarsest, CG) .. top, in one block (q1_bottom.cu):
     // A[1 .. top] Q1 grid operators of at most 33 points per line that q1_bottom_fits

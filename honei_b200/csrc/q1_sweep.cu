@@ -34,29 +34,24 @@ namespace hb2
     static int find_grid_typed(hb2_ell_s * A, uint32_t m, cudaStream_t stream)
     {
         const EllView<T> V = A->view<T>();
+        // the stream's workspace holds the row and the flag (no allocation, no device-wide wait)
+        Workspace * ws = 0;
+        int st = stream_workspace(stream, &ws);
+        if (st) return st;
         T ref[10];
-        char * d = 0;
-        HB2_CUDA(cudaMalloc(&d, 10 * sizeof(T) + sizeof(int) + 8));
-        T * dref = (T *)d;
-        int * dbad = (int *)(d + 10 * sizeof(T));
-        cudaError_t e = cudaMemsetAsync(dbad, 0, sizeof(int), stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(dref, sizeof(T), V.val + m + 1, V.ld * sizeof(T), sizeof(T), 9,
-                                  cudaMemcpyDeviceToDevice, stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(dref + 9, V.val, sizeof(T), cudaMemcpyDeviceToDevice, stream);
+        T * dref = (T *)(ws->scalars + 32);
+        int * dbad = (int *)(ws->scalars + 44);
+        HB2_CUDA(cudaMemsetAsync(dbad, 0, sizeof(int), stream));
+        HB2_CUDA(cudaMemcpy2DAsync(dref, sizeof(T), V.val + m + 1, V.ld * sizeof(T), sizeof(T), 9,
+                                   cudaMemcpyDeviceToDevice, stream));
+        HB2_CUDA(cudaMemcpyAsync(dref + 9, V.val, sizeof(T), cudaMemcpyDeviceToDevice, stream));
+        q1_grid_check_kernel<T><<<ceil_div(A->rows, 256), 256, 0, stream>>>(V, m, dref, dbad);
+        count_launches(1);
+        HB2_LAUNCH_CHECK("Q1 grid check");
         int bad = 1;
-        if (e == cudaSuccess)
-        {
-            q1_grid_check_kernel<T><<<ceil_div(A->rows, 256), 256, 0, stream>>>(V, m, dref, dbad);
-            count_launches(1);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(ref, dref, sizeof(ref), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        cudaFree(d);
-        if (e != cudaSuccess) return cuda_status(e, "Q1 grid check");
+        HB2_CUDA(cudaMemcpyAsync(ref, dref, sizeof(ref), cudaMemcpyDeviceToHost, stream));
+        HB2_CUDA(cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        HB2_CUDA(cudaStreamSynchronize(stream));
         if (bad) return HB2_OK;
         for (int k = 0; k < 9; ++k) A->q1g_v[k] = (double)ref[k];
         A->q1g_vb = (double)ref[9];
@@ -96,6 +91,8 @@ namespace hb2
         g.cb = (T *)p.coarse_b;
         g.cz = (T *)p.coarse_zero;
         g.partials = p.ws ? p.ws->partials : nullptr;
+        g.y32 = p.y32;
+        g.z32 = p.z32;
         g.list = p.list;
         g.count = p.count;
         g.vs = p.vstride;
@@ -111,7 +108,7 @@ namespace hb2
 
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream)
     {
-        if (! A->q1g_m || p.sweeps < 1 || p.sweeps > kQ1SweepMax) return fail(HB2_ERR_UNSUPPORTED, "Q1 sweep");
+        if (! A->q1g_m || p.sweeps < (sweep_single(p.tail) ? 0 : 1) || p.sweeps > kQ1SweepMax) return fail(HB2_ERR_UNSUPPORTED, "Q1 sweep");
         SweepLaunch l;
         l.nvec = p.list ? p.nvec : 1;
         l.max_vec = p.list ? p.max_vec : 1;
@@ -120,5 +117,51 @@ namespace hb2
         l.blocks = p.blocks;
         l.stream = stream;
         return A->dtype == HB2_F64 ? launch_typed<double>(A, p, l) : launch_typed<float>(A, p, l);
+    }
+
+    // Product, defect (+ norm) and product with dot of a large Q1 grid operator as streaming
+    // passes.  From 2^16 rows up: below, the one-row-per-thread kernels are as fast and their
+    // layout was timed at creation.  Measured (B200), FP64 level 11: defect + norm 37.2 us
+    // with the gather kernel.
+    bool q1_single_applies(const hb2_ell_s * A, int mode)
+    {
+        return A->q1g_m >= 257 && (mode == kPlain || mode == kDefect || mode == kDot);
+    }
+
+    int launch_q1_single(const hb2_ell_s * A, int mode, const void * x, void * y, const void * b, double * red,
+                         int want_sqrt, const Workspace * ws, cudaStream_t stream)
+    {
+        Q1SweepPass p;
+        unsigned blocks = 0;
+        p.tail = mode == kPlain ? kSweepProduct : (mode == kDefect ? kSweepDefect : kSweepDot);
+        p.x = x;
+        p.b = b;
+        p.y = y;
+        p.ws = red ? ws : nullptr;
+        p.blocks = &blocks;
+        const int st = launch_q1_sweep(A, p, stream);
+        if (st || ! red) return st;
+        launch_sum_partials(ws->partials, blocks, 1, red, want_sqrt, stream);
+        HB2_LAUNCH_CHECK("Q1 pass: partials");
+        return HB2_OK;
+    }
+
+    int launch_q1_ir_defect(const hb2_ell_s * A, const double * x, const double * b, float * b32, float * x32,
+                            double * red, const Workspace * ws, cudaStream_t stream)
+    {
+        Q1SweepPass p;
+        unsigned blocks = 0;
+        p.tail = kSweepDefectIR;
+        p.x = x;
+        p.b = b;
+        p.y32 = b32;
+        p.z32 = x32;
+        p.ws = ws;
+        p.blocks = &blocks;
+        const int st = launch_q1_sweep(A, p, stream);
+        if (st) return st;
+        launch_sum_partials(ws->partials, blocks, 1, red, 1, stream);
+        HB2_LAUNCH_CHECK("IR defect: partials");
+        return HB2_OK;
     }
 }

@@ -41,7 +41,16 @@
 namespace hb2
 {
     enum { kSweepLoad = 0, kSweepZero = 1 };                            // HEAD
-    enum { kSweepStore = 0, kSweepRestrict = 1, kSweepNorm = 2 };       // TAIL
+    // TAIL; the last four without sweeps (S = 0): y = b - A x (+ ||y||^2), y = A x (+ <y, x>),
+    // and the refinement's defect, rounded to FP32 into y32 with z32 cleared (+ ||b - A x||^2)
+    enum { kSweepStore = 0, kSweepRestrict = 1, kSweepNorm = 2, kSweepDefect = 3, kSweepProduct = 4, kSweepDot = 5,
+           kSweepDefectIR = 6 };
+    __host__ __device__ constexpr bool sweep_single(int tail) { return tail >= kSweepDefect; }
+    __host__ __device__ constexpr bool sweep_reads_b(int tail) { return tail != kSweepProduct && tail != kSweepDot; }
+    __host__ __device__ constexpr bool sweep_reduces(int tail)
+    {
+        return tail == kSweepNorm || tail == kSweepDefect || tail == kSweepDot || tail == kSweepDefectIR;
+    }
 
     template <typename T>
     struct Q1SweepArgs
@@ -56,7 +65,8 @@ namespace hb2
         T * y;                  // iterate out, != x
         T * cb;                 // kSweepRestrict: coarser right-hand side
         T * cz;                 // kSweepRestrict: coarser vector cleared on the way (nullable)
-        double * partials;      // kSweepNorm: one partial per block
+        double * partials;      // reducing tails: one partial per block (nullable but for kSweepNorm)
+        float * y32, * z32;     // kSweepDefectIR (z32 nullable)
         int strips, chunks, rows;   // strips of columns x chunks of `rows` rows
         int bpv;                // blocks per vector
         // batched: vectors list[0 .. *count), the fine arrays vs elements apart, the coarse ones cs
@@ -137,7 +147,7 @@ namespace hb2
         const int m = g.m;
         pdl_entry();
         T Pi = T(0), Pb = T(0);
-        if (! PVEC) { Pb = __ldg(g.jac); Pi = __ldg(g.jac + m + 1); }
+        if (! PVEC && ! sweep_single(TAIL)) { Pb = __ldg(g.jac); Pi = __ldg(g.jac + m + 1); }
         const uint32_t nblk = g.list ? *g.count * (uint32_t)g.bpv : gridDim.x;
         double part = 0.0;
         for (uint32_t blk = blockIdx.x; blk < nblk; blk += gridDim.x)
@@ -172,9 +182,9 @@ namespace hb2
             }
             // rows kb .. ke of x, b (P, c) into the rings, D rows ahead
             const T * xg = HEAD == kSweepLoad ? g.x + vo : nullptr;
-            const T * bg = g.b + vo;
+            const T * bg = sweep_reads_b(TAIL) ? g.b + vo : nullptr;
             const T * pg = PVEC ? g.jac : nullptr;
-            const T * cg = (HEAD == kSweepLoad && g.c) ? g.c + co : nullptr;
+            const T * cg = (HEAD == kSweepLoad && ! sweep_single(TAIL) && g.c) ? g.c + co : nullptr;
             const int cbase = base >> 1;
             auto fetch_coarse = [&](int I) {
                 for (int j = lane; j < K::CW; j += 32)
@@ -187,7 +197,7 @@ namespace hb2
             // running pointers of the next row to fetch (this lane's first column)
             const int64_t fo = (int64_t)kb * m + base + lane;
             const T * xf = HEAD == kSweepLoad ? xg + fo : nullptr;
-            const T * bf = bg + fo;
+            const T * bf = sweep_reads_b(TAIL) ? bg + fo : nullptr;
             const T * pf = PVEC ? pg + fo : nullptr;
             bool in[C];
 #pragma unroll
@@ -200,13 +210,13 @@ namespace hb2
                     for (int q = 0; q < C; ++q)
                         if (in[q])
                         {
-                            cp_async_elem<sizeof(T)>(br + 32 * q, bf + 32 * q);
+                            if (sweep_reads_b(TAIL)) cp_async_elem<sizeof(T)>(br + 32 * q, bf + 32 * q);
                             if (HEAD == kSweepLoad) cp_async_elem<sizeof(T)>(xr + 32 * q, xf + 32 * q);
                             if (PVEC) cp_async_elem<sizeof(T)>(pring + (f & RBM) * W + lane + 32 * q, pf + 32 * q);
                         }
                     if (HEAD == kSweepLoad && cg && (f & 1)) fetch_coarse((f + 1) >> 1);
                 }
-                bf += m;
+                if (sweep_reads_b(TAIL)) bf += m;
                 if (HEAD == kSweepLoad) xf += m;
                 if (PVEC) pf += m;
                 cp_async_commit();
@@ -226,7 +236,7 @@ namespace hb2
             for (int c = 0; c < C; ++c) cur[NA][c] = racc[c] = T(0);
 
             // running pointer of the row the last sweep completes in the next step
-            constexpr int YLAG = NSM > 0 ? 2 * NSM - 1 : 0;
+            constexpr int YLAG = NSM > 0 ? 2 * NSM - 1 : (sweep_single(TAIL) ? 1 : 0);
             T * yr = g.y + vo + col0 + ((int64_t)kb - YLAG) * m;
             const T * brl = bring + lane * C, * prl = pring + lane * C;
                         auto step = [&](auto interior, auto parity, int s) {
@@ -327,19 +337,19 @@ namespace hb2
                 {
                     const int q = s - 2 * t - 1;                 // the row this stage completes
                     T bq[C];
-                    lds_vec<T, C>(bq, brl + (q & RBM) * W);
+                    if (sweep_reads_b(TAIL)) lds_vec<T, C>(bq, brl + (q & RBM) * W);
 #pragma unroll
                     for (int c = 0; c < C; ++c)
                     {
                         if ((! IN && (q == 0 || q == m - 1)) || edge[c]) ax[t][c] = M::fma(g.vb, xprev[t][c], T(0));
-                        res[t][c] = M::sub(bq[c], ax[t][c]);
+                        res[t][c] = sweep_reads_b(TAIL) ? M::sub(bq[c], ax[t][c]) : ax[t][c];
                     }
                 }
 #pragma unroll
                 for (int t = NS - 1; t >= 0; --t)
                 {
                     const int q = s - 2 * t - 1;
-                    T out[C];
+                    T out[C], xq[C];
                     if (t < NSM)
                     {
                         T pq[C];
@@ -357,7 +367,11 @@ namespace hb2
                         for (int c = 0; c < C; ++c) out[c] = res[t][c];
                     }
 #pragma unroll
-                    for (int c = 0; c < C; ++c) xprev[t][c] = cur[t][c];
+                    for (int c = 0; c < C; ++c)
+                    {
+                        xq[c] = xprev[t][c];
+                        xprev[t][c] = cur[t][c];
+                    }
                     if (t < NSM)
                     {
 #pragma unroll
@@ -376,6 +390,26 @@ namespace hb2
 #pragma unroll
                             for (int c = 0; c < C; ++c)
                                 if (own[c]) part = fma((double)out[c], (double)out[c], part);
+                        }
+                    }
+                    else if (sweep_single(TAIL))
+                    {
+                        if (q >= r0 && q < r1)
+                        {
+#pragma unroll
+                            for (int c = 0; c < C; ++c)
+                                if (own[c])
+                                {
+                                    if (TAIL == kSweepDefectIR)
+                                    {
+                                        const int64_t o = (int64_t)q * m + col0 + c;
+                                        g.y32[o] = (float)out[c];
+                                        if (g.z32) g.z32[o] = 0.f;
+                                    }
+                                    else yr[c] = out[c];
+                                    if (sweep_reduces(TAIL))
+                                        part = fma((double)out[c], (double)(TAIL == kSweepDot ? xq[c] : out[c]), part);
+                                }
                         }
                     }
                     else if (TAIL == kSweepRestrict)
@@ -442,7 +476,7 @@ namespace hb2
             }
             cp_async_wait<0>();
         }
-        if (TAIL == kSweepNorm)
+        if (sweep_reduces(TAIL) && g.partials)
         {
             __shared__ double scratch[32];
             const double sum = block_sum(part, scratch);
@@ -481,7 +515,7 @@ namespace hb2
         typedef Q1SweepShape<T, C, S, HEAD, TAIL> K;
         g.strips = (g.m + K::WV - 1) / K::WV;
         g.rows = sweep_chunk_rows(g.m, g.strips, K::HALO, K::NS, sweep_blocks_per_sm<T, C>(), nvec);
-        if (TAIL == kSweepNorm)
+        if (sweep_reduces(TAIL) && g.partials)
             while ((uint64_t)g.strips * ((g.m + g.rows - 1) / g.rows) / kSweepWarps + 1 > max_partials) g.rows *= 2;   // even stays even
         g.chunks = (g.m + g.rows - 1) / g.rows;
         g.bpv = (g.strips * g.chunks + kSweepWarps - 1) / kSweepWarps;

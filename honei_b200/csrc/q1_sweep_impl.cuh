@@ -39,12 +39,30 @@ namespace hb2
         return q1_sweep_s<T, C, UNI, kSweepLoad, kSweepStore, false>(g, S, l);
     }
 
+    // the passes without sweeps, on the wide form
+    template <typename T, int C, bool UNI>
+    static int q1_single(const Q1SweepArgs<T> & g, int tail, const SweepLaunch & l)
+    {
+#define HB2_SG(TAIL_) q1_sweep_launch_one<T, C, UNI, 0, kSweepLoad, TAIL_, false>(g, l.nvec, l.max_vec, l.cap, l.max_partials, l.blocks, l.stream)
+        switch (tail)
+        {
+            case kSweepDefect: return HB2_SG(kSweepDefect);
+            case kSweepProduct: return HB2_SG(kSweepProduct);
+            case kSweepDot: return HB2_SG(kSweepDot);
+            default:
+                if constexpr (sizeof(T) == 8) return HB2_SG(kSweepDefectIR);
+                else return fail(HB2_ERR_UNSUPPORTED, "Q1 pass");
+        }
+#undef HB2_SG
+    }
+
     // CW columns a lane when wide, else CN (equal: one form); the general nine-value form
     // and the given Jacobi vector (pvec) run wide only
     template <typename T, int CW, int CN>
     static int q1_sweep_typed(const Q1SweepArgs<T> & g, bool wide, bool uni, int S, int head, int tail, bool pvec,
                               const SweepLaunch & l)
     {
+        if (sweep_single(tail)) return uni ? q1_single<T, CW, true>(g, tail, l) : q1_single<T, CW, false>(g, tail, l);
         if (pvec)
             return uni ? q1_sweep_s<T, CW, true, kSweepLoad, kSweepStore, true>(g, S, l)
                        : q1_sweep_s<T, CW, false, kSweepLoad, kSweepStore, true>(g, S, l);
