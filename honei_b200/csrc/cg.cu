@@ -481,7 +481,11 @@ extern "C" int hb2_cg_solve(hb2_ell A, const void * b, void * x, uint64_t max_it
     HB2_CUDA(cudaMemsetAsync(ws->scalars + 8, 0, 2 * sizeof(double), stream));
     const size_t es = dtype_size(A->dtype), n = A->rows;
     if (n == 0) { if (used_iters) *used_iters = 0; if (final_defect) *final_defect = 0; return HB2_OK; }
-    if (cg_small_fits(A) && n <= 4096)
+    // a Q1 grid operator that fits a cluster; otherwise one block, or the whole GPU
+    st = cg_cluster_applies(A) ? launch_cg_cluster(A, b, x, max_iters, eps, used_dev, def_dev, stream)
+                               : HB2_ERR_UNSUPPORTED;
+    if (st == HB2_OK) {}
+    else if (cg_small_fits(A) && n <= 4096)
     {
         st = launch_cg_small(A, b, x, max_iters, eps, 0, used_dev, def_dev, stream);
         if (st) return st;

@@ -426,6 +426,11 @@ namespace hb2
     int launch_cg_small(const hb2_ell_s * A, const void * b, void * x, uint64_t max_iters, double eps, int exact,
                         uint64_t * used_dev, double * defect_dev, cudaStream_t stream);
     bool cg_small_fits(const hb2_ell_s * A);
+    // CG of a Q1 grid operator on one cluster (cg_cluster.cu); HB2_ERR_UNSUPPORTED when it
+    // cannot be resident
+    bool cg_cluster_applies(const hb2_ell_s * A);
+    int launch_cg_cluster(const hb2_ell_s * A, const void * b, void * x, uint64_t max_iters, double eps,
+                          uint64_t * used_dev, double * defect_dev, cudaStream_t s);
     bool cg_mixed_supported(const hb2_ell_s * A64);
     int launch_cg_small_f32io(const hb2_ell_s * A64, const void * b32, void * x32, uint64_t max_iters, double eps,
                               int exact, uint64_t * used_dev, double * defect_dev, cudaStream_t stream);
