@@ -22,6 +22,9 @@
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
 
+#include "cg_warp.cuh"
+
+#include <algorithm>
 #include <cfloat>
 #include <cstring>
 
@@ -147,6 +150,263 @@ namespace
         const double ta = st->alpha_new / eps_guard(st->alpha);
         for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
             p[i] = __dadd_rn(__dmul_rn(p[i], ta), __dmul_rn(d[i], r[i]));
+    }
+
+    // ------------------------------------------------------------------
+    // CG with a vector P, the whole loop in one cooperative launch.
+    //
+    // Up to some hundred thousand rows an iteration as four graph nodes (product and dot,
+    // update and dots, decision, direction) spends most of its time between the kernels, on
+    // their ramps, tickets and on vectors read and written back.  Here one block per SM stays
+    // resident with its rows of x, r, p and d in shared memory and of v in registers, only the
+    // matrix (which the L2 holds) and p move, and the kernels' ends become three grid barriers.
+    // The rounding of every update is that of the separate kernels; the dots are summed per
+    // block and then over the blocks in a fixed order, by every warp alike, so all blocks take
+    // the same decisions.  Measured (B200, 491,401 rows of nine stored entries, 200 steps):
+    // 41 us a step as graph nodes.
+    constexpr int kLoopThreads = 512;
+    constexpr int kLoopRows = 13;       // rows a thread: four vectors of them in 227 KB
+
+    struct LoopArgs
+    {
+        EllView<double> A;
+        uint32_t m;                     // Q1 grid operator (q1g_m): its rows from the grid
+        double a[9], ab;
+        uint32_t n, rows;               // rows per thread
+        uint64_t max_iters;
+        double eps;
+        int smoother;
+        double * x, * p;
+        const double * r, * d;
+        KState * st;
+        double * partials;              // 3 x gridDim
+        unsigned * arrived;             // zero at launch
+        int * error;
+    };
+
+    // all blocks have arrived; a wait of more than a second ends with an error flag
+    __device__ __forceinline__ bool loop_barrier(const LoopArgs & g, unsigned target, int * ok)
+    {
+        if (threadIdx.x == 0)
+        {
+            __threadfence();
+            atomicAdd(g.arrived, 1u);
+            *ok = 1;
+            unsigned long long t0 = 0;
+            for (unsigned spin = 0;; ++spin)
+            {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.arrived) : "memory");
+                if (v >= target) break;
+                if ((spin & 1023u) == 1023u)
+                {
+                    const unsigned long long t = global_ns();
+                    if (t0 == 0) t0 = t;
+                    if (t - t0 > 1000000000ull || *((volatile int *)g.error) != 0)
+                    {
+                        atomicExch(g.error, 1);
+                        *ok = 0;
+                        break;
+                    }
+                }
+            }
+            __threadfence();
+        }
+        __syncthreads();
+        return *ok != 0;
+    }
+
+    // KT: 9 slots unrolled, 0 any number, -1 the Q1 grid
+    template <int KT>
+    __device__ __forceinline__ double loop_row(const LoopArgs & g, uint32_t row, const double * p)
+    {
+        double s = 0.0;
+        if constexpr (KT == -1)
+        {
+            const uint32_t m = g.m, i = row / m, j = row - i * m;
+            if (i == 0 || j == 0 || i == m - 1 || j == m - 1) return __dadd_rn(0.0, __dmul_rn(g.ab, p[row]));
+            const double * c = p + row;
+            double xv[9];
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+            {
+                xv[q] = c[-(int)m + (q - 1)];
+                xv[3 + q] = c[q - 1];
+                xv[6 + q] = c[(int)m + (q - 1)];
+            }
+#pragma unroll
+            for (int q = 0; q < 9; ++q) s = __dadd_rn(s, __dmul_rn(g.a[q], xv[q]));
+        }
+        else if constexpr (KT > 0)
+        {
+            double a[KT], xv[KT];
+            int c[KT];
+#pragma unroll
+            for (int k = 0; k < KT; ++k)
+            {
+                c[k] = __ldg(g.A.col + (uint64_t)k * g.A.ld + row);
+                a[k] = __ldg(g.A.val + (uint64_t)k * g.A.ld + row);
+            }
+#pragma unroll
+            for (int k = 0; k < KT; ++k) xv[k] = c[k] >= 0 ? p[c[k]] : 0.0;
+#pragma unroll
+            for (int k = 0; k < KT; ++k)
+                if (c[k] >= 0) s = __dadd_rn(s, __dmul_rn(a[k], xv[k]));
+        }
+        else
+        {
+            for (uint32_t k = 0; k < g.A.K; ++k)
+            {
+                const int c = __ldg(g.A.col + (uint64_t)k * g.A.ld + row);
+                if (c >= 0) s = __dadd_rn(s, __dmul_rn(__ldg(g.A.val + (uint64_t)k * g.A.ld + row), p[c]));
+            }
+        }
+        return s;
+    }
+
+    template <int KT, int E>
+    __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(const __grid_constant__ LoopArgs g)
+    {
+        extern __shared__ double loop_smem[];
+        __shared__ double wred[2][kLoopThreads / 32];
+        __shared__ int ok;
+        const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+        const uint32_t cap = g.rows * kLoopThreads, row0 = blockIdx.x * cap + t;
+        double * xs = loop_smem + t, * rs = xs + cap, * ps = rs + cap, * ds = ps + cap;
+        double v[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+        {
+            const uint32_t row = row0 + e * kLoopThreads;
+            v[e] = 0.0;
+            if (e < (int)g.rows && row < g.n)
+            {
+                xs[e * kLoopThreads] = g.x[row];
+                rs[e * kLoopThreads] = g.r[row];
+                ps[e * kLoopThreads] = g.p[row];
+                ds[e * kLoopThreads] = g.d[row];
+            }
+        }
+        unsigned target = 0;
+        double alpha_new = g.st->alpha_new;
+        const double init = g.st->init;
+        double cur = 0.0;
+        unsigned long long it = 0, used = 0;
+        // sums a0 (and a1) over all blocks, the same in every thread
+        // (the one-value and the two-value sums have partials of their own: a block may write
+        // the next ones while another still reads these)
+        auto total = [&](double & a0, double & a1, bool two) -> bool {
+            double * part = g.partials + (two ? gridDim.x : 0);
+            a0 = warp_sum_mma(a0);
+            if (two) a1 = warp_sum_mma(a1);
+            if (lane == 0)
+            {
+                wred[0][warp] = a0;
+                wred[1][warp] = a1;
+            }
+            __syncthreads();
+            if (warp == 0)
+            {
+                const double s0 = warp_sum_mma(lane < kLoopThreads / 32 ? wred[0][lane] : 0.0);
+                const double s1 = two ? warp_sum_mma(lane < kLoopThreads / 32 ? wred[1][lane] : 0.0) : 0.0;
+                if (lane == 0)
+                {
+                    part[blockIdx.x] = s0;
+                    if (two) part[gridDim.x + blockIdx.x] = s1;
+                }
+            }
+            target += gridDim.x;
+            if (! loop_barrier(g, target, &ok)) return false;
+            double s0 = 0.0, s1 = 0.0;
+            for (unsigned b = lane; b < gridDim.x; b += 32)
+            {
+                s0 += __ldcg(part + b);
+                if (two) s1 += __ldcg(part + gridDim.x + b);
+            }
+            a0 = warp_sum_mma(s0);
+            if (two) a1 = warp_sum_mma(s1);
+            return true;
+        };
+        while (true)
+        {
+            // v = A p, <v, p>
+            double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+            {
+                const uint32_t row = row0 + e * kLoopThreads;
+                if (e < (int)g.rows && row < g.n)
+                {
+                    v[e] = loop_row<KT>(g, row, g.p);
+                    a0 = fma(v[e], ps[e * kLoopThreads], a0);
+                }
+            }
+            if (! total(a0, a1, false)) return;
+            // x += lambda p, r -= lambda v, <d r, r>, ||r||^2
+            const double lambda = alpha_new / eps_guard(a0), ml = -lambda;
+            a0 = a1 = 0.0;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+            {
+                const uint32_t row = row0 + e * kLoopThreads;
+                if (e < (int)g.rows && row < g.n)
+                {
+                    xs[e * kLoopThreads] = axpy(lambda, ps[e * kLoopThreads], xs[e * kLoopThreads]);
+                    const double ri = axpy(ml, v[e], rs[e * kLoopThreads]);
+                    rs[e * kLoopThreads] = ri;
+                    a0 = fma(__dmul_rn(ds[e * kLoopThreads], ri), ri, a0);
+                    a1 = fma(ri, ri, a1);
+                }
+            }
+            if (! total(a0, a1, true)) return;
+            ++it;
+            bool stop;
+            if (g.smoother) stop = it == g.max_iters;
+            else
+            {
+                cur = sqrt(a1);
+                stop = cur < g.eps * init || cur < g.eps || it == g.max_iters;
+            }
+            if (stop) { used = it; break; }
+            // p = p talpha + d r
+            const double ta = a0 / eps_guard(alpha_new);
+            alpha_new = a0;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+            {
+                const uint32_t row = row0 + e * kLoopThreads;
+                if (e < (int)g.rows && row < g.n)
+                {
+                    const double pv = __dadd_rn(__dmul_rn(ps[e * kLoopThreads], ta),
+                                                __dmul_rn(ds[e * kLoopThreads], rs[e * kLoopThreads]));
+                    ps[e * kLoopThreads] = pv;
+                    g.p[row] = pv;
+                }
+            }
+            __syncthreads();
+            target += gridDim.x;
+            if (! loop_barrier(g, target, &ok)) return;
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+        {
+            const uint32_t row = row0 + e * kLoopThreads;
+            if (e < (int)g.rows && row < g.n) g.x[row] = xs[e * kLoopThreads];
+        }
+        if (blockIdx.x == 0 && t == 0)
+        {
+            g.st->iter = it;
+            g.st->used = used;
+            g.st->cur = cur;
+        }
+    }
+
+    __global__ void k_cg_loop_init(KState * st, unsigned * arrived, int * error)
+    {
+        *error = 0;
+        st->iter = 0;
+        st->used = 0;
+        *arrived = 0;
     }
 
     __global__ void k_cg_init(KState * st, uint64_t max_iters, cudaGraphConditionalHandle h)
@@ -441,6 +701,70 @@ namespace
         return HB2_OK;
     }
 
+    // CG with a vector P whose rows fit the resident blocks, on a matrix read from its plain
+    // arrays or the grid (other layouts move fewer bytes as kernels of their own)
+    bool loop_applies(const hb2_krylov_s * K)
+    {
+        return K->method != HB2_BICGSTAB_VAR && K->pdiag && K->max_iters > 0 && K->n >= 2048 &&
+               K->n <= (uint64_t)kLoopThreads * kLoopRows * num_sms() && (K->A->q1g_m || K->A->layout[1] == kLayoutPlain);
+    }
+
+    template <int KT, int E>
+    cudaError_t launch_loop_e(const LoopArgs & g, cudaStream_t s)
+    {
+        const size_t smem = 4 * sizeof(double) * (size_t)g.rows * kLoopThreads;
+        cudaError_t e = cudaFuncSetAttribute(k_cg_loop<KT, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ceil_div(g.n, (uint64_t)g.rows * kLoopThreads));
+        cfg.blockDim = dim3(kLoopThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_cg_loop<KT, E>, g);
+    }
+
+    template <int KT>
+    cudaError_t launch_loop(const LoopArgs & g, cudaStream_t s)
+    {
+        return g.rows <= 2   ? launch_loop_e<KT, 2>(g, s)
+               : g.rows <= 4 ? launch_loop_e<KT, 4>(g, s)
+               : g.rows <= 8 ? launch_loop_e<KT, 8>(g, s)
+                             : launch_loop_e<KT, kLoopRows>(g, s);
+    }
+
+    int record_loop(hb2_krylov_s * K, cudaStream_t s)
+    {
+        LoopArgs g = {};
+        g.A = K->A->view<double>();
+        g.m = K->A->q1g_m;
+        for (int k = 0; k < 9; ++k) g.a[k] = K->A->q1g_v[k];
+        g.ab = K->A->q1g_vb;
+        g.n = (uint32_t)K->n;
+        g.rows = ceil_div(K->n, (uint64_t)kLoopThreads * num_sms());
+        g.max_iters = K->max_iters;
+        g.eps = K->eps;
+        g.smoother = K->method == HB2_CG_SMOOTHER;
+        g.x = K->v(1);
+        g.r = K->v(2);
+        g.p = K->v(3);
+        g.d = K->pdiag;
+        g.st = K->st;
+        g.partials = K->ws->partials;
+        g.arrived = K->ws->bar_words;
+        g.error = K->ws->error;
+        k_cg_loop_init<<<1, 1, 0, s>>>(K->st, g.arrived, g.error);
+        const cudaError_t e = g.m ? launch_loop<-1>(g, s) : K->A->K == 9 ? launch_loop<9>(g, s) : launch_loop<0>(g, s);
+        count_launches(2);
+        if (e != cudaSuccess) return cuda_status(e, "krylov CG loop");
+        HB2_LAUNCH_CHECK("krylov CG loop");
+        return HB2_OK;
+    }
+
     int body_cg(hb2_krylov_s * K, cudaGraphConditionalHandle h_loop)
     {
         const uint64_t n = K->n;
@@ -573,6 +897,18 @@ namespace
         return HB2_OK;
     }
 
+    int finish_graph(hb2_krylov_s * K, uint64_t before)
+    {
+        cudaGraph_t g = nullptr;
+        cudaError_t ce = cudaStreamEndCapture(K->cap, &g);
+        set_launch_count(before);
+        if (ce != cudaSuccess) return cuda_status(ce, "cudaStreamEndCapture (krylov)");
+        K->graph = g;
+        ce = cudaGraphInstantiate(&K->exec, g, 0);
+        if (ce != cudaSuccess) return cuda_status(ce, "cudaGraphInstantiate (krylov)");
+        return HB2_OK;
+    }
+
     int build_graph(hb2_krylov_s * K)
     {
         const uint64_t before = hb2_launch_count();
@@ -587,8 +923,9 @@ namespace
         size_t ndeps = 0;
         cudaError_t ce = cudaStreamGetCaptureInfo(K->cap, &cs, 0, &capg, &deps, &ndeps);
         if (ce != cudaSuccess) return capture_fail(K, ce, "cudaStreamGetCaptureInfo");
-        cudaGraphConditionalHandle h_loop;
-        ce = cudaGraphConditionalHandleCreate(&h_loop, capg, 0, 0);
+        cudaGraphConditionalHandle h_loop = {};
+        const bool loop = loop_applies(K);
+        if (! loop) ce = cudaGraphConditionalHandleCreate(&h_loop, capg, 0, 0);
         if (ce != cudaSuccess) return capture_fail(K, ce, "cudaGraphConditionalHandleCreate");
         if (K->method == HB2_BICGSTAB_VAR)
         {
@@ -604,14 +941,26 @@ namespace
                 if (K->pdiag) e = precond(K, r, p, r, &st->alpha_new, nullptr, nullptr, nullptr, nullptr, K->cap);
                 else e = launch_ell(K->P, kDot, r, p, 0, 0, 0, &st->alpha_new, 0, K->ws, K->cap);
             }
+            if (! e && loop) e = record_loop(K, K->cap);
             if (e) { capture_fail(K, cudaSuccess, ""); return e; }
-            k_cg_init<<<1, 1, 0, K->cap>>>(st, K->max_iters, h_loop);
-            count_launches(1);
+            if (! loop)
+            {
+                k_cg_init<<<1, 1, 0, K->cap>>>(st, K->max_iters, h_loop);
+                count_launches(1);
+            }
         }
         ce = cudaGetLastError();
         if (ce == cudaSuccess) ce = cudaStreamGetCaptureInfo(K->cap, &cs, 0, &capg, &deps, &ndeps);
         if (ce != cudaSuccess) return capture_fail(K, ce, "capture (prefix)");
         K->prefix_kernels = hb2_launch_count() - before;
+        if (loop)
+        {
+            ce = cudaMemcpyAsync(K->host_st, st, sizeof(KState), cudaMemcpyDeviceToHost, K->cap);
+            if (ce == cudaSuccess)
+                ce = cudaMemcpyAsync(K->ws->host_scalars, K->ws->error, sizeof(int), cudaMemcpyDeviceToHost, K->cap);
+            if (ce != cudaSuccess) return capture_fail(K, ce, "state copy");
+            return finish_graph(K, before);
+        }
         cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
         cp.conditional.handle = h_loop;
         cp.conditional.type = cudaGraphCondTypeWhile;
@@ -635,14 +984,7 @@ namespace
         if (ce != cudaSuccess) return capture_fail(K, ce, "state copy");
         (void)n;
         (void)p;
-        cudaGraph_t g = nullptr;
-        ce = cudaStreamEndCapture(K->cap, &g);
-        set_launch_count(before);
-        if (ce != cudaSuccess) return cuda_status(ce, "cudaStreamEndCapture (krylov)");
-        K->graph = g;
-        ce = cudaGraphInstantiate(&K->exec, g, 0);
-        if (ce != cudaSuccess) return cuda_status(ce, "cudaGraphInstantiate (krylov)");
-        return HB2_OK;
+        return finish_graph(K, before);
     }
 
     void krylov_free(hb2_krylov_s * K)
@@ -726,6 +1068,9 @@ extern "C" int hb2_krylov_solve(hb2_krylov K, const void * b, void * x, uint64_t
     if (st) return st;
     HB2_CUDA(cudaStreamSynchronize(stream));
     const KState & h = *K->host_st;
+    int herr = 0;
+    if (K->body_kernels == 0 && K->method != HB2_BICGSTAB_VAR) memcpy(&herr, K->ws->host_scalars, sizeof(int));
+    if (herr) return fail(HB2_ERR_TIMEOUT, "hb2_krylov_solve: a grid barrier wait expired");
     uint64_t used;
     double defect;
     if (K->method == HB2_BICGSTAB_VAR)

@@ -1,0 +1,84 @@
+"""The resident forms of the conjugate-gradient solvers: CGSolver NONE on a Q1 grid
+operator as one cluster (csrc/cg_cluster.cu, math/cg.hh:64-135) and CGSolver VAR with a
+vector P as one cooperative launch (csrc/krylov.cu, math/cg.hh:142-210), at the sizes
+where their splits change.  The dots are summed in another order than the reference's, so
+a solve may stop a step earlier or later and is held to its own stopping test."""
+import numpy as np
+import pytest
+import torch
+
+import honei_b200 as hb
+from honei_b200 import DenseVector, SparseMatrixELL
+from honei_b200.inputs import q1_coefficient_operator, uniform
+
+pytestmark = pytest.mark.gpu
+
+
+def dvec(a):
+    return DenseVector(torch.from_numpy(np.ascontiguousarray(a)).cuda())
+
+
+# one CTA with 1 and 2 nodes a thread (levels 4, 5), 4 and 16 CTAs with 2 and 9 (6, 7, 8)
+@pytest.mark.parametrize("level", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("aniso", [1.0, 2.0])
+def test_cluster_cg(oracle, level, aniso):
+    ref = oracle.q1_ell(level, aniso=aniso)
+    b = oracle.ell_spmv(ref, oracle.uniform(ref.rows, 42))
+    x0 = 0.1 * oracle.uniform(ref.rows, 7)
+    A = SparseMatrixELL.poisson_q1(level, aniso=aniso)
+    for start in (np.zeros(ref.rows), x0):
+        x = dvec(start)
+        _, used, defect = hb.CGSolver.value(A, None, dvec(b), x, 3000, 1e-8)
+        _, ref_used = oracle.cg_q1(level, b, x0=start, max_iters=3000, aniso=aniso)[:2]
+        r0 = np.linalg.norm(b - oracle.ell_spmv(ref, start))
+        assert abs(used - ref_used) <= 1
+        # the recursive residual meets the test; the true one follows it to well within a half
+        assert defect < 1e-8 * r0
+        assert np.linalg.norm(b - oracle.ell_spmv(ref, x.numpy())) < 1.5e-8 * r0
+
+
+@pytest.mark.parametrize("level", [4, 7, 8])
+@pytest.mark.parametrize("cap", [0, 1, 5])
+def test_cluster_cg_caps(oracle, level, cap):
+    """After a few steps the iterates agree to rounding: a step's sums of n terms, at most
+    n eps off, change the iterate by that much relative to its size."""
+    ref = oracle.q1_ell(level)
+    b = oracle.ell_spmv(ref, oracle.uniform(ref.rows, 42))
+    x = dvec(np.zeros(ref.rows))
+    _, used, _ = hb.CGSolver.value(SparseMatrixELL.poisson_q1(level), None, dvec(b), x, cap, 1e-8)
+    xo = oracle.cg_q1(level, b, max_iters=cap)[0]
+    assert used == cap
+    assert np.linalg.norm(x.numpy() - xo) <= 2.0 ** -52 * ref.rows * max(1.0, np.linalg.norm(xo))
+
+
+def test_cluster_cg_f32():
+    """FP32 vectors, FP64 dots: the true residual in FP64 is within FP32 rounding of the stop."""
+    level, m = 6, 65
+    A = SparseMatrixELL.poisson_q1(level, torch.float32)
+    b = dvec(uniform(m * m, 3, dtype=np.float32))
+    x = DenseVector(m * m, dtype=torch.float32)
+    hb.CGSolver.value(A, None, b, x, 2000, 1e-4)
+    r = DenseVector(m * m, dtype=torch.float32)
+    hb.Defect.value(r, b, A, x)
+    # 1e-4 by the recursion, 1e-4 again for its drift over some 200 steps of 6e-8
+    assert hb.Norm.value(r) < 2e-4 * hb.Norm.value(b)
+
+
+# rows a thread: 1 (one block of 5), 1, 2 and 3
+@pytest.mark.parametrize("cells", [47, 100, 350, 449])
+@pytest.mark.parametrize("cap", [1, 40])
+def test_cg_var_loop(oracle, cells, cap):
+    op = q1_coefficient_operator(np.power(4.0, uniform(cells * cells, 5, -0.5, 0.5)).reshape(cells, cells))
+    n = op[0]
+    ref = oracle.Ell(n, n, op[2], op[3], 1, *op[4:])
+    A = SparseMatrixELL.from_arrays(*op)
+    P = oracle.jacobi_vector(ref)
+    b = oracle.ell_spmv(ref, uniform(n, 42))
+    x, used, _ = hb.KrylovSolver(hb.HB2_CG_VAR, A, dvec(P), cap, 0.0).solve(dvec(b), dvec(np.zeros(n)))
+    xo, ref_used = oracle.cg_var(ref, P, b, max_iters=cap, eps=0.0)[:2]
+    assert used == ref_used == cap
+    # dots of n terms in another order: n eps a step, over `cap` steps
+    assert np.linalg.norm(x.numpy() - xo) <= 2.0 ** -52 * n * cap * np.linalg.norm(xo)
+    s = hb.CGSmoother.value(A, dvec(P), dvec(b), dvec(np.zeros(n)), cap)
+    so = oracle.cg_var(ref, P, b, max_iters=cap, eps=0.0, smoother=True)[0]
+    assert np.linalg.norm(s.numpy() - so) <= 2.0 ** -52 * n * cap * np.linalg.norm(so)
