@@ -41,10 +41,10 @@ namespace hb2
     {
         double d0, d1, e0, e1;
         const double one = 1.0, zero = 0.0;
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
                      : "=d"(d0), "=d"(d1) : "d"(one), "d"(v), "d"(zero), "d"(zero));
         const double s = d0 + d1;
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
                      : "=d"(e0), "=d"(e1) : "d"(s), "d"(one), "d"(zero), "d"(zero));
         return e0;
     }
@@ -219,6 +219,7 @@ namespace hb2
             const T thr = M::mul(eps, initial), thr2 = M::mul(thr, thr), eps2 = M::mul(eps, eps);
 #pragma unroll
             for (int j = 0; j < RPL; ++j) sr[j] = wr[j];
+            const T inv_eps = Recip<T>::rn(Eps<T>::v());
             T * cur = sp, * nxt = sp2;
             while (it < max_iters)
             {
@@ -229,40 +230,45 @@ namespace hb2
                     if (lane + 32 * j < n) nxt[lane + 32 * j] = rr[j];
                 }
                 __syncwarp();
-#pragma unroll
-                for (int j = 0; j < RPL; ++j) xr[j] = M::fma(a, pr[j], xr[j]);
-                spmv_tree(wr, nxt);
-                T * t = cur;
-                cur = nxt;
-                nxt = t;
+                // ||r||^2 while the product's gathers are on their way
                 double s1 = 0.0, s2 = 0.0;
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
                     if (lane + 32 * j < n) s1 = fma((double)rr[j], (double)rr[j], s1);
                 const T g = (T)warp_sum_mma(s1);
+                spmv_tree(wr, nxt);
+#pragma unroll
+                for (int j = 0; j < RPL; ++j) xr[j] = M::fma(a, pr[j], xr[j]);
+                T * t = cur;
+                cur = nxt;
+                nxt = t;
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
                     if (lane + 32 * j < n) s2 = fma((double)wr[j], (double)rr[j], s2);
                 del = (T)warp_sum_mma(s2);
                 ++it;
-                if (g < thr2 || g < eps2 || it == max_iters)
-                {
-                    current = sqrt(g);
-                    used = it;
-                    break;
-                }
-                // single-rounded reciprocals instead of IEEE divisions (this mode is
-                // not the reference's order anyway); 1/g and b do not wait for (w, r)
+                // single-rounded reciprocals instead of IEEE divisions (this mode is not the
+                // reference's order anyway).  A warp issues in order, so what the next step
+                // needs is formed before the sum (w, r) arrives -- b, 1/g and with them p and s --
+                // and 1/a as t/g, not by a third reciprocal behind a
                 const T b = M::mul(g, inv_g), bg = M::mul(M::mul(b, g), inv_a);
-                inv_g = Recip<T>::rn(guard(g));
-                a = M::mul(g, Recip<T>::rn(guard(M::sub(del, bg))));
+                const T ig = Recip<T>::rn(guard(g));
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
                 {
                     pr[j] = M::fma(b, pr[j], rr[j]);
                     sr[j] = M::fma(b, sr[j], wr[j]);
                 }
-                inv_a = Recip<T>::rn(guard(a));
+                if (g < thr2 || g < eps2 || it == max_iters)
+                {
+                    current = sqrt(g);
+                    used = it;
+                    break;
+                }
+                const T d = guard(M::sub(del, bg));
+                a = M::mul(g, Recip<T>::rn(d));
+                inv_g = ig;
+                inv_a = fabs(a) > Eps<T>::v() ? M::mul(d, ig) : inv_eps;
             }
             it = max_iters;   // done: skip the loop below
         }

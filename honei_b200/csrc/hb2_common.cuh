@@ -278,7 +278,7 @@ namespace hb2
     __device__ __forceinline__ T q1_prolong_row(uint64_t r, const T * c, uint32_t mf, uint32_t mc)
     {
         typedef Arith<T> M;
-        const uint32_t i = (uint32_t)(r / mf), j = (uint32_t)(r - (uint64_t)i * mf);
+        const uint32_t i = (uint32_t)r / mf, j = (uint32_t)r - i * mf;     // grids of less than 2^32 nodes
         const T * cp = c + (uint64_t)(i >> 1) * mc + (j >> 1);
         const T h = T(0.5), q = T(0.25);
         if (! (i & 1) && ! (j & 1)) return M::add(T(0), M::mul(T(1), q1_load<T, L2>(cp)));
@@ -293,7 +293,7 @@ namespace hb2
     __device__ __forceinline__ T q1_restrict_row(uint64_t r, const T * x, uint32_t mf, uint32_t mc)
     {
         typedef Arith<T> M;
-        const int I = (int)(r / mc), J = (int)(r - (uint64_t)I * mc);
+        const int I = (int)((uint32_t)r / mc), J = (int)((uint32_t)r - (uint32_t)I * mc);
         T acc = T(0);
 #pragma unroll
         for (int di = -1; di <= 1; ++di)

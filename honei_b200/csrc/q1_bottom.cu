@@ -54,74 +54,111 @@ namespace hb2
         }
     };
 
-    // A x of the thread's rows, x in shared memory
-    template <typename T>
-    __device__ __forceinline__ void bottom_product(const BottomLevel<T> & L, const BottomNodes & o, const T * x,
-                                                   T (&ax)[kBottomRows], T (&xc)[kBottomRows])
+    // A x of R rows from the thread's first one, x in shared memory.  Without branches: rows
+    // and columns outside the grid read a clamped neighbour and boundary rows are selected at
+    // the end, so the chains of all rows run side by side.  UNI: all couplings equal, one
+    // product per value.
+    template <typename T, bool UNI, int R>
+    __device__ __forceinline__ void bottom_product(const BottomLevel<T> & L, const BottomNodes & o, const T * x, T (&ax)[R],
+                                                   T (&xc)[R])
     {
         typedef Arith<T> M;
+        const int jw = max(o.j - 1, 0), je = min(o.j + 1, o.m - 1);
         const bool ecol = o.j == 0 || o.j == o.m - 1;
-        T w[3], c[3], e[3];                 // rows i - 1, i, i + 1
-        auto load = [&](int k, int i) {
-            const bool ok = i >= 0 && i < o.m;
-            const T * r = x + i * o.m + o.j;
-            w[k] = ok && ! ecol ? r[-1] : T(0);
-            c[k] = ok ? r[0] : T(0);
-            e[k] = ok && ! ecol ? r[1] : T(0);
-        };
-        if (o.rows == 0) return;
-        load(0, o.i0 - 1);
-        load(1, o.i0);
+        T w[R + 2], c[R + 2], e[R + 2], pc[R + 2];
 #pragma unroll
-        for (int k = 0; k < kBottomRows; ++k)
+        for (int k = 0; k < R + 2; ++k)
         {
-            if (k >= o.rows) break;
-            const int i = o.i0 + k;
-            load((k + 2) % 3, i + 1);
-            const int a = k % 3, b = (k + 1) % 3, d = (k + 2) % 3;
-            xc[k] = c[b];
-            if (ecol || i == 0 || i == o.m - 1) ax[k] = M::add(T(0), M::mul(L.vb, c[b]));
+            const T * r = x + min(max(o.i0 + k - 1, 0), o.m - 1) * o.m;
+            w[k] = r[jw];
+            c[k] = r[o.j];
+            e[k] = r[je];
+        }
+        if (UNI)
+        {
+#pragma unroll
+            for (int k = 0; k < R + 2; ++k)
+            {
+                w[k] = M::fma(L.v[0], w[k], T(0));      // the sum 0 + p of the first slot folded in
+                pc[k] = M::fma(L.v[0], c[k], T(0));
+                e[k] = M::fma(L.v[0], e[k], T(0));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+        {
+            T s;
+            if (UNI)
+            {
+                s = M::add(M::add(w[k], pc[k]), e[k]);
+                s = M::add(M::add(M::add(s, w[k + 1]), M::mul(L.v[4], c[k + 1])), e[k + 1]);
+                s = M::add(M::add(M::add(s, w[k + 2]), pc[k + 2]), e[k + 2]);
+            }
             else
             {
-                T s = M::add(T(0), M::mul(L.v[0], w[a]));
-                s = M::add(s, M::mul(L.v[1], c[a]));
-                s = M::add(s, M::mul(L.v[2], e[a]));
-                s = M::add(s, M::mul(L.v[3], w[b]));
-                s = M::add(s, M::mul(L.v[4], c[b]));
-                s = M::add(s, M::mul(L.v[5], e[b]));
-                s = M::add(s, M::mul(L.v[6], w[d]));
-                s = M::add(s, M::mul(L.v[7], c[d]));
-                ax[k] = M::add(s, M::mul(L.v[8], e[d]));
+                s = M::add(T(0), M::mul(L.v[0], w[k]));
+                s = M::add(s, M::mul(L.v[1], c[k]));
+                s = M::add(s, M::mul(L.v[2], e[k]));
+                s = M::add(s, M::mul(L.v[3], w[k + 1]));
+                s = M::add(s, M::mul(L.v[4], c[k + 1]));
+                s = M::add(s, M::mul(L.v[5], e[k + 1]));
+                s = M::add(s, M::mul(L.v[6], w[k + 2]));
+                s = M::add(s, M::mul(L.v[7], c[k + 2]));
+                s = M::add(s, M::mul(L.v[8], e[k + 2]));
             }
+            const int i = o.i0 + k;
+            xc[k] = c[k + 1];
+            ax[k] = ecol || i == 0 || i >= o.m - 1 ? M::add(T(0), M::mul(L.vb, c[k + 1])) : s;
         }
     }
 
-    // `sweeps` Jacobi sweeps from x0 (in shared memory) with ping-pong into x1; returns the
-    // buffer that holds the result
-    template <typename T>
-    __device__ __forceinline__ T * bottom_smooth(const BottomLevel<T> & L, const BottomNodes & o, T * x0, T * x1, const T * b,
-                                                 int sweeps)
+    // `sweeps` Jacobi sweeps from x0 (in shared memory) with ping-pong into x1, and with
+    // DEFECT the defect of the result into the buffer that is then free; returns the buffer
+    // that holds the result
+    template <typename T, bool UNI, int R, bool DEFECT>
+    __device__ __forceinline__ T * bottom_smooth_r(const BottomLevel<T> & L, const BottomNodes & o, T * x0, T * x1,
+                                                   const T * b, int sweeps)
     {
         typedef Arith<T> M;
         const T Pi = L.jac[L.m + 1], Pb = L.jac[0];
+        const bool ecol = o.j == 0 || o.j == o.m - 1;
+        T rhs[R], P[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+        {
+            const int i = o.i0 + k;
+            rhs[k] = k < o.rows ? b[i * o.m + o.j] : T(0);
+            P[k] = ecol || i == 0 || i == o.m - 1 ? Pb : Pi;
+        }
+        T ax[R], xc[R];
         for (int s = 0; s < sweeps; ++s)
         {
-            T ax[kBottomRows], xc[kBottomRows];
-            bottom_product(L, o, x0, ax, xc);
+            bottom_product<T, UNI, R>(L, o, x0, ax, xc);
 #pragma unroll
-            for (int k = 0; k < kBottomRows; ++k)
-                if (k < o.rows)
-                {
-                    const int i = o.i0 + k, q = i * o.m + o.j;
-                    const T P = i == 0 || i == o.m - 1 || o.j == 0 || o.j == o.m - 1 ? Pb : Pi;
-                    x1[q] = M::add(xc[k], M::mul(P, M::sub(b[q], ax[k])));
-                }
+            for (int k = 0; k < R; ++k)
+                if (k < o.rows) x1[(o.i0 + k) * o.m + o.j] = M::add(xc[k], M::mul(P[k], M::sub(rhs[k], ax[k])));
             __syncthreads();
             T * t = x0;
             x0 = x1;
             x1 = t;
         }
+        if (DEFECT)
+        {
+            bottom_product<T, UNI, R>(L, o, x0, ax, xc);
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+                if (k < o.rows) x1[(o.i0 + k) * o.m + o.j] = M::sub(rhs[k], ax[k]);
+            __syncthreads();
+        }
         return x0;
+    }
+
+    template <typename T, bool UNI, bool DEFECT>
+    __device__ __forceinline__ T * bottom_smooth(const BottomLevel<T> & L, T * x0, T * x1, const T * b, int sweeps)
+    {
+        const BottomNodes o(L.m);
+        return L.m > 2 * (kBottomThreads / L.m) ? bottom_smooth_r<T, UNI, kBottomRows, DEFECT>(L, o, x0, x1, b, sweeps)
+                                                : bottom_smooth_r<T, UNI, 2, DEFECT>(L, o, x0, x1, b, sweeps);
     }
 
     template <typename TA, typename S>
@@ -136,7 +173,7 @@ namespace hb2
         }
     }
 
-    template <typename T, bool MIXED>
+    template <typename T, bool MIXED, bool UNI>
     __global__ void __launch_bounds__(kBottomThreads, 1) q1_bottom_kernel(const __grid_constant__ BottomArgs<T> g)
     {
         typedef Arith<T> M;
@@ -168,19 +205,8 @@ namespace hb2
                     xs[l][q] = g.zero_guess ? T(0) : g.x[q];
                 }
             __syncthreads();
-            const BottomNodes o(L.m);
-            T * cur = bottom_smooth(L, o, xs[l], ts[l], bs[l], g.n_pre);
+            T * cur = bottom_smooth<T, UNI, true>(L, xs[l], ts[l], bs[l], g.n_pre);
             T * r = cur == xs[l] ? ts[l] : xs[l];
-            T ax[kBottomRows], xc[kBottomRows];
-            bottom_product(L, o, cur, ax, xc);
-#pragma unroll
-            for (int k = 0; k < kBottomRows; ++k)
-                if (k < o.rows)
-                {
-                    const int q = (o.i0 + k) * o.m + o.j;
-                    r[q] = M::sub(bs[l][q], ax[k]);
-                }
-            __syncthreads();
             const int mc = g.lev[l - 1].m;
             for (int q = threadIdx.x; q < mc * mc; q += kBottomThreads)
             {
@@ -208,8 +234,7 @@ namespace hb2
             for (int q = threadIdx.x; q < n; q += kBottomThreads)
                 xs[l][q] = M::add(xs[l][q], q1_prolong_row<T, false>(q, xs[l - 1], L.m, g.lev[l - 1].m));
             __syncthreads();
-            const BottomNodes o(L.m);
-            xs[l] = bottom_smooth(L, o, xs[l], ts[l], bs[l], g.n_post);
+            xs[l] = bottom_smooth<T, UNI, false>(L, xs[l], ts[l], bs[l], g.n_post);
             if (l == g.top)
                 for (int q = threadIdx.x; q < n; q += kBottomThreads) g.x[q] = xs[l][q];
         }
@@ -249,8 +274,13 @@ namespace hb2
         g.used = p.used;
         g.defect = p.defect;
         const size_t smem = (3 * 96 + 2) * sizeof(double) + elems * sizeof(T);
-        if (p.coarse64) launch_pdl(q1_bottom_kernel<T, true>, dim3(1), dim3(kBottomThreads), smem, s, g);
-        else launch_pdl(q1_bottom_kernel<T, false>, dim3(1), dim3(kBottomThreads), smem, s, g);
+        bool uni = true;
+        for (int l = 1; l <= p.top; ++l)
+            for (int k = 0; k < 9; ++k) uni = uni && (k == 4 || p.A[l]->q1g_v[k] == p.A[l]->q1g_v[0]);
+#define HB2_BOTTOM(M_, U_) launch_pdl(q1_bottom_kernel<T, M_, U_>, dim3(1), dim3(kBottomThreads), smem, s, g)
+        if (p.coarse64) { if (uni) HB2_BOTTOM(true, true); else HB2_BOTTOM(true, false); }
+        else { if (uni) HB2_BOTTOM(false, true); else HB2_BOTTOM(false, false); }
+#undef HB2_BOTTOM
         count_launches(1);
         HB2_LAUNCH_CHECK("V-cycle bottom launch");
         return HB2_OK;
