@@ -19,6 +19,7 @@
 // reference, and the norm (a tree reduction) only decides when to stop.
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
+#include "transfer_free.cuh"
 
 #include <cfloat>
 #include <cmath>
@@ -69,11 +70,11 @@ namespace
 
     // x = x + alpha c with alpha = <d, c> / <A c, c> in the vectors' type
     template <typename T>
-    __global__ void k_axpy_adaptive(T * x, const T * c, const double * dots, uint64_t n)
+    __global__ void k_axpy_adaptive(T * out, const T * x, const T * c, const double * dots, uint64_t n)
     {
         const T alpha = Arith<T>::div((T)dots[0], (T)dots[1]);
         for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-            x[i] = Arith<T>::add(x[i], Arith<T>::mul(alpha, c[i]));
+            out[i] = Arith<T>::add(x[i], Arith<T>::mul(alpha, c[i]));
     }
 
     template <typename T>
@@ -134,8 +135,8 @@ namespace
     // math/conjugate_gradients.hh:491-560 with the banded cg_kernel (:108-151); the
     // loop runs while ||x||^2 grows by more than konv_rad (at most `cap` steps)
     template <typename T>
-    __global__ void k_coarse_cg(const T * bands, uint64_t n, uint64_t m, const T * rhs, T * x, T * g, T * u, T * e,
-                                T * ng, double konv_rad, uint64_t cap, LState * st)
+    __device__ void coarse_cg_thread(const T * bands, uint64_t n, uint64_t m, const T * rhs, T * x, T * g, T * u, T * e,
+                                     T * ng, double konv_rad, uint64_t cap, LState * st)
     {
         typedef Arith<T> M;
         const T eps = Eps<T>::v();
@@ -163,6 +164,205 @@ namespace
             norm_x_last = norm_x;
             norm_x = seq_dot(x, x, n);
             ++it;
+        }
+    }
+
+    // The same with at most 32 unknowns in one full warp, lane = row: the products of all rows
+    // side by side in each row's own order, the dots one chain over the lanes' values in every
+    // lane alike -- the same bits.  The level-1 grid's nine unknowns: one thread walks 81
+    // dependent terms a product, two products and four dots a step.
+    template <typename T>
+    __device__ void coarse_cg_warp(const T * bands, int n, int m, const T * rhs, T * xout, double konv_rad, uint64_t cap,
+                                   LState * st)
+    {
+        typedef Arith<T> M;
+        const T eps = Eps<T>::v();
+        const int i = threadIdx.x & 31;
+        const bool ok = i < n;
+        const int off[9] = {-m - 1, -m, -m + 1, -1, 0, 1, m - 1, m, m + 1};
+        T a[9];
+#pragma unroll
+        for (int b = 0; b < 9; ++b) a[b] = ok ? bands[(int64_t)b * n + i] : T(0);
+        auto product = [&](T v) -> T {
+            T s = M::mul(a[4], v);
+#pragma unroll
+            for (int b = 0; b < 9; ++b)
+            {
+                const int j = i + off[b];
+                const T w = __shfl_sync(0xffffffffu, v, j & 31);
+                if (b != 4 && j >= 0 && j < n) s = M::add(s, M::mul(a[b], w));
+            }
+            return s;
+        };
+        auto dot = [&](T v, T w) -> T {
+            T s = T(0);
+            for (int k = 0; k < n; ++k)
+                s = M::fma(__shfl_sync(0xffffffffu, v, k), __shfl_sync(0xffffffffu, w, k), s);
+            return s;
+        };
+        const T r = ok ? rhs[i] : T(0);
+        T x = T(0), g = M::sub(product(x), r), u = M::mul(g, T(-1));
+        T norm_x = dot(x, x), norm_x_last = M::sub(norm_x, T(1));
+        uint64_t it = 0;
+        while ((double)M::sub(norm_x, norm_x_last) > konv_rad)
+        {
+            if (it == cap) { if (i == 0) st->err = 1; break; }
+            T upper = dot(g, g);
+            T e = product(u);
+            T lower = dot(e, u);
+            T f = fabs(lower) >= eps ? M::div(upper, lower) : M::div(upper, eps);
+            e = M::add(M::mul(u, f), x);
+            lower = upper;
+            const T ng = M::sub(product(e), r);
+            upper = dot(ng, ng);
+            f = fabs(lower) >= eps ? M::div(upper, lower) : M::div(upper, eps);
+            u = M::sub(M::mul(u, f), ng);
+            g = ng;
+            x = e;
+            norm_x_last = norm_x;
+            norm_x = dot(x, x);
+            ++it;
+        }
+        if (ok) xout[i] = x;
+    }
+
+    template <typename T>
+    __global__ void k_coarse_cg(const T * bands, uint64_t n, uint64_t m, const T * rhs, T * x, T * g, T * u, T * e,
+                                T * ng, double konv_rad, uint64_t cap, LState * st)
+    {
+        if (n <= 32) coarse_cg_warp(bands, (int)n, (int)m, rhs, x, konv_rad, cap, st);
+        else if (threadIdx.x == 0) coarse_cg_thread(bands, n, m, rhs, x, g, u, e, ng, konv_rad, cap, st);
+    }
+
+    // out = x + alpha P c in one pass (the prolonged correction, math/prolongation.hh, then
+    // ScaledSum)
+    template <typename T>
+    __global__ void k_prolong_axpy(T * out, const T * x, const T * coarse, T alpha, uint64_t n, uint64_t m, Mask mk)
+    {
+        for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+            out[i] = Arith<T>::add(x[i], Arith<T>::mul(alpha, free_prolong_node(coarse, i, m, mk)));
+    }
+
+    // ------------------------------------------------------------------
+    // The levels of at most 33 x 33 points below the finest, the coarsest solve among them,
+    // in one block: as kernels of their own each level took about ten launches of 2.5 us a
+    // cycle and the coarse CG 15 us in one thread.  The level vectors live in shared memory,
+    // the bands stay in L1; a phase is one block barrier.  Not with the adaptive correction,
+    // whose dots are grid reductions.
+    constexpr int kLBottomLevels = 6, kLBottomThreads = 512;
+    constexpr uint64_t kLBottomRows = 33 * 33;
+
+    template <typename T>
+    struct LBottom
+    {
+        struct
+        {
+            const T * bands, * dinv;
+            int n, m;
+        } lev[kLBottomLevels];
+        int top;
+        uint64_t npre;
+        T alpha;
+        const T * rhs;          // of level top
+        T * x;                  // of level top
+        T * cg;                 // scratch of the one-thread coarse CG
+        double konv_rad;
+        Mask mk;
+        LState * st;
+    };
+
+    template <typename T, int MODE>
+    __device__ __forceinline__ void lb_apply(const T * bands, int n, int m, const T * x, T * y, const T * rhs, const T * dinv)
+    {
+        typedef Arith<T> M;
+        const int off[9] = {-m - 1, -m, -m + 1, -1, 0, 1, m - 1, m, m + 1};
+        for (int i = threadIdx.x; i < n; i += kLBottomThreads)
+        {
+            T a[9];
+#pragma unroll
+            for (int b = 0; b < 9; ++b) a[b] = __ldg(bands + b * n + i);
+            T s = M::mul(a[4], x[i]);
+#pragma unroll
+            for (int b = 0; b < 9; ++b)
+            {
+                if (b == 4) continue;
+                const int j = i + off[b];
+                if (j >= 0 && j < n) s = M::add(s, M::mul(a[b], x[j]));
+            }
+            if (MODE == 1) y[i] = M::sub(rhs[i], s);
+            else y[i] = M::add(x[i], M::mul(M::sub(rhs[i], s), __ldg(dinv + i)));
+        }
+        __syncthreads();
+    }
+
+    template <typename T>
+    __global__ void __launch_bounds__(kLBottomThreads) k_lmg_bottom(const __grid_constant__ LBottom<T> g)
+    {
+        typedef Arith<T> M;
+        extern __shared__ __align__(16) unsigned char lb_smem[];
+        T * mem = reinterpret_cast<T *>(lb_smem);
+        T * x[kLBottomLevels], * t[kLBottomLevels], * r[kLBottomLevels];     // iterate, other buffer, rhs
+#pragma unroll
+        for (int l = 0; l < kLBottomLevels; ++l)
+        {
+            const int n = l <= g.top ? g.lev[l].n : 0;
+            x[l] = mem;
+            t[l] = mem + n;
+            r[l] = mem + 2 * n;
+            mem += 3 * n;
+        }
+#pragma unroll
+        for (int l = kLBottomLevels - 1; l >= 1; --l)
+        {
+            if (l > g.top) continue;
+            const auto & L = g.lev[l];
+            if (l == g.top)
+            {
+                for (int i = threadIdx.x; i < L.n; i += kLBottomThreads) r[l][i] = g.rhs[i];
+                __syncthreads();
+            }
+            for (int i = threadIdx.x; i < L.n; i += kLBottomThreads) x[l][i] = M::mul(__ldg(L.dinv + i), r[l][i]);
+            __syncthreads();
+            for (uint64_t k = 0; k + 1 < g.npre; ++k)
+            {
+                lb_apply<T, 2>(L.bands, L.n, L.m, x[l], t[l], r[l], L.dinv);
+                T * q = x[l];
+                x[l] = t[l];
+                t[l] = q;
+            }
+            lb_apply<T, 1>(L.bands, L.n, L.m, x[l], t[l], r[l], nullptr);
+            for (int i = threadIdx.x; i < g.lev[l - 1].n; i += kLBottomThreads)
+                r[l - 1][i] = free_restrict_node(t[l], (uint64_t)i, (uint64_t)L.m, g.mk);
+            __syncthreads();
+        }
+        {
+            const auto & C = g.lev[0];
+            if (C.n <= 32)
+            {
+                if (threadIdx.x < 32) coarse_cg_warp(C.bands, C.n, C.m, r[0], x[0], g.konv_rad, 100000, g.st);
+            }
+            else if (threadIdx.x == 0)
+                coarse_cg_thread(C.bands, (uint64_t)C.n, (uint64_t)C.m, (const T *)r[0], x[0], g.cg, g.cg + C.n, g.cg + 2 * C.n,
+                                 g.cg + 3 * C.n, g.konv_rad, 100000, g.st);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int l = 1; l < kLBottomLevels; ++l)
+        {
+            if (l > g.top) continue;
+            const auto & L = g.lev[l];
+            for (int i = threadIdx.x; i < L.n; i += kLBottomThreads)
+                x[l][i] = M::add(x[l][i], M::mul(g.alpha, free_prolong_node(x[l - 1], (uint64_t)i, (uint64_t)L.m, g.mk)));
+            __syncthreads();
+            for (uint64_t k = 0; k < g.npre; ++k)
+            {
+                lb_apply<T, 2>(L.bands, L.n, L.m, x[l], t[l], r[l], L.dinv);
+                T * q = x[l];
+                x[l] = t[l];
+                t[l] = q;
+            }
+            if (l == g.top)
+                for (int i = threadIdx.x; i < L.n; i += kLBottomThreads) g.x[i] = x[l][i];
         }
     }
 
@@ -232,17 +432,63 @@ struct hb2_lmg_s
 
 namespace
 {
+    // k Jacobi sweeps that end in v: they start from v, or from L.tmp when k is odd
+    // (sweeps_start), so no copy follows
+    void * sweeps_start(hb2_lmg_s::Level & L, void * v, uint64_t k) { return k & 1 ? L.tmp : v; }
+
     template <typename T>
     int sweeps(hb2_lmg_s * G, hb2_lmg_s::Level & L, void * v, const void * rhs, uint64_t k, cudaStream_t s)
     {
-        void * cur = v, * nxt = L.tmp;
+        void * cur = sweeps_start(L, v, k), * nxt = k & 1 ? v : L.tmp;
         for (uint64_t i = 0; i < k; ++i)
         {
             int st = launch_q1(L.A, 2, cur, nxt, rhs, L.dinv, G->ws->error, s);
             if (st) return st;
             std::swap(cur, nxt);
         }
-        if (cur != v) return launch_copy(G->dtype, v, cur, L.n, s);
+        return HB2_OK;
+    }
+
+    // the highest level the bottom kernel takes (below the finest), 0: none
+    int bottom_top(const hb2_lmg_s * G)
+    {
+        const int nl = (int)(G->lmax - G->lmin) + 1;
+        if (G->prm.adaptive && G->prm.adapt_correction_factor == 0.0) return 0;
+        if (G->prm.n_pre_smooth < 1) return 0;
+        int t = 0;
+        for (int i = 0; i + 1 < nl && i < kLBottomLevels && G->lev[i].n <= kLBottomRows; ++i) t = i;
+        return t;
+    }
+
+    template <typename T>
+    int launch_bottom(hb2_lmg_s * G, int top, cudaStream_t s)
+    {
+        LBottom<T> g = {};
+        size_t elems = 0;
+        for (int i = 0; i <= top; ++i)
+        {
+            auto & L = G->lev[i];
+            g.lev[i].bands = (const T *)L.A->bands;
+            g.lev[i].dinv = (const T *)L.dinv;
+            g.lev[i].n = (int)L.n;
+            g.lev[i].m = (int)L.m;
+            elems += 3 * L.n;
+        }
+        g.top = top;
+        g.npre = G->prm.n_pre_smooth;
+        g.alpha = (T)G->prm.adapt_correction_factor;
+        g.rhs = (const T *)G->lev[top].rhs;
+        g.x = (T *)G->lev[top].x;
+        g.cg = (T *)G->cg;
+        g.konv_rad = (double)std::numeric_limits<T>::epsilon();
+        g.mk = make_mask(G->prm.macro_border_mask);
+        g.st = G->st;
+        const size_t smem = elems * sizeof(T);
+        if (smem > 48 * 1024)
+            HB2_CUDA(cudaFuncSetAttribute(k_lmg_bottom<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_lmg_bottom<T><<<1, kLBottomThreads, smem, s>>>(g);
+        count_launches(1);
+        HB2_LAUNCH_CHECK("lmg bottom");
         return HB2_OK;
     }
 
@@ -258,20 +504,21 @@ namespace
         int st = HB2_OK;
         if (nl == 1)
         {
-            k_coarse_cg<T><<<1, 1, 0, s>>>((const T *)C.A->bands, C.n, C.m, (const T *)C.d, (T *)C.x, cgv, cgv + nc,
+            k_coarse_cg<T><<<1, 32, 0, s>>>((const T *)C.A->bands, C.n, C.m, (const T *)C.d, (T *)C.x, cgv, cgv + nc,
                                            cgv + 2 * nc, cgv + 3 * nc, (double)std::numeric_limits<T>::epsilon(),
                                            100000, G->st);
             count_launches(1);
             HB2_LAUNCH_CHECK("lmg coarse cg");
             return launch_q1(C.A, 1, C.x, C.d, C.rhs, nullptr, G->ws->error, s);
         }
-        for (int i = (int)nl - 1; i >= 1 && ! st; --i)
+        const int bottom = bottom_top(G);
+        for (int i = (int)nl - 1; i > bottom && ! st; --i)
         {
             auto & L = G->lev[i];
             const uint32_t g = grid_of(L.n);
             if (i == (int)nl - 1)
             {
-                k_eprod<T><<<g, 256, 0, s>>>((T *)L.c, (const T *)L.dinv, (const T *)L.d, L.n);
+                k_eprod<T><<<g, 256, 0, s>>>((T *)sweeps_start(L, L.c, npre - 1), (const T *)L.dinv, (const T *)L.d, L.n);
                 count_launches(1);
                 HB2_LAUNCH_CHECK("lmg jacobi start");
                 st = sweeps<T>(G, L, L.c, L.d, npre - 1, s);
@@ -282,7 +529,7 @@ namespace
             }
             else
             {
-                k_eprod<T><<<g, 256, 0, s>>>((T *)L.x, (const T *)L.dinv, (const T *)L.rhs, L.n);
+                k_eprod<T><<<g, 256, 0, s>>>((T *)sweeps_start(L, L.x, npre - 1), (const T *)L.dinv, (const T *)L.rhs, L.n);
                 count_launches(1);
                 HB2_LAUNCH_CHECK("lmg jacobi start");
                 st = sweeps<T>(G, L, L.x, L.rhs, npre - 1, s);
@@ -294,36 +541,47 @@ namespace
                                      G->prm.macro_border_mask, s);
         }
         if (st) return st;
-        k_coarse_cg<T><<<1, 1, 0, s>>>((const T *)C.A->bands, C.n, C.m, (const T *)C.rhs, (T *)C.x, cgv, cgv + nc,
-                                       cgv + 2 * nc, cgv + 3 * nc, (double)std::numeric_limits<T>::epsilon(), 100000,
-                                       G->st);
-        count_launches(1);
-        HB2_LAUNCH_CHECK("lmg coarse cg");
-        for (unsigned i = 1; i < nl && ! st; ++i)
+        if (bottom > 0) st = launch_bottom<T>(G, bottom, s);
+        else
+        {
+            k_coarse_cg<T><<<1, 32, 0, s>>>((const T *)C.A->bands, C.n, C.m, (const T *)C.rhs, (T *)C.x, cgv, cgv + nc,
+                                            cgv + 2 * nc, cgv + 3 * nc, (double)std::numeric_limits<T>::epsilon(),
+                                            100000, G->st);
+            count_launches(1);
+            HB2_LAUNCH_CHECK("lmg coarse cg");
+        }
+        if (st) return st;
+        for (unsigned i = (unsigned)bottom + 1; i < nl && ! st; ++i)
         {
             auto & L = G->lev[i];
-            st = hb2_prolongation((hb2_dtype)G->dtype, L.c, L.n, G->lev[i - 1].x, G->lev[i - 1].n,
-                                  G->prm.macro_border_mask, s);
-            if (st) break;
-            if (G->prm.adaptive && G->prm.adapt_correction_factor == 0.0)
+            const bool adaptive = G->prm.adaptive && G->prm.adapt_correction_factor == 0.0;
+            if (adaptive)
             {
+                st = hb2_prolongation((hb2_dtype)G->dtype, L.c, L.n, G->lev[i - 1].x, G->lev[i - 1].n,
+                                      G->prm.macro_border_mask, s);
+                if (st) break;
                 // math/multigrid.hh:1712-1721 (the MIXED kernel): alpha = <d, c> / <A c, c>
                 double * dots = G->st->dots[G->lmin + i];
                 st = launch_q1(L.A, 0, L.c, L.tmp, nullptr, nullptr, G->ws->error, s);
                 if (st) break;
                 k_dot2<T><<<grid_of(L.n), 256, 0, s>>>((const T *)L.d, (const T *)L.c, (const T *)L.tmp, L.n,
                                                        G->ws->slot(), dots);
-                k_axpy_adaptive<T><<<grid_of(L.n), 256, 0, s>>>((T *)L.x, (const T *)L.c, dots, L.n);
+                k_axpy_adaptive<T><<<grid_of(L.n), 256, 0, s>>>((T *)sweeps_start(L, L.x, npre), (const T *)L.x,
+                                                                (const T *)L.c, dots, L.n);
                 count_launches(2);
             }
             else
             {
-                k_axpy<T><<<grid_of(L.n), 256, 0, s>>>((T *)L.x, (const T *)L.c, alpha, L.n);
+                k_prolong_axpy<T><<<grid_of(L.n), 256, 0, s>>>((T *)sweeps_start(L, L.x, npre), (const T *)L.x,
+                                                               (const T *)G->lev[i - 1].x, alpha, L.n, L.m,
+                                                               make_mask(G->prm.macro_border_mask));
                 count_launches(1);
             }
             HB2_LAUNCH_CHECK("lmg correction");
             st = sweeps<T>(G, L, L.x, L.rhs, npre, s);
-            if (! st) st = launch_q1(L.A, 1, L.x, L.d, L.rhs, nullptr, G->ws->error, s);
+            // the defect is read by the finest level's norm and next cycle; a coarser level forms
+            // its own again on the next way down before anything reads it
+            if (! st && i == nl - 1) st = launch_q1(L.A, 1, L.x, L.d, L.rhs, nullptr, G->ws->error, s);
         }
         return st;
     }

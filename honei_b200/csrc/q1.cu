@@ -113,26 +113,41 @@ namespace hb2
         }
     }
 
-    // plain-load variant for x pointers that are not 16-byte aligned
+    // Plain-load variant: one row a thread, every load of the row issued before the first
+    // product.  For x pointers that are not 16-byte aligned, and for the grids up to
+    // kQ1GatherRows rows, where the three window copies of a block, which complete one after
+    // another (about 0.6 us each), cost more than the nine gathers.
+    constexpr uint64_t kQ1GatherRows = 1u << 19;
+
     template <typename T, int MODE>
-    __global__ void q1_kernel_direct(const T * __restrict__ bands, const T * __restrict__ x, T * __restrict__ y,
-                                     const T * __restrict__ rhs, const T * __restrict__ dinv, int64_t n, int64_t m)
+    __global__ void __launch_bounds__(256) q1_kernel_direct(const T * __restrict__ bands, const T * __restrict__ x,
+                                                            T * __restrict__ y, const T * __restrict__ rhs,
+                                                            const T * __restrict__ dinv, int64_t n, int64_t m)
     {
         typedef Arith<T> M;
         const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (i >= n) return;
         const int64_t off[9] = {-m - 1, -m, -m + 1, -1, 0, 1, m - 1, m, m + 1};
-        T s = M::mul(bands[4 * n + i], x[i]);
+        T a[9], xv[9];
+#pragma unroll
         for (int b = 0; b < 9; ++b)
         {
-            if (b == 4) continue;
             const int64_t j = i + off[b];
-            if (j < 0 || j >= n) continue;
-            s = M::add(s, M::mul(bands[b * n + i], __ldg(x + j)));
+            a[b] = __ldg(bands + b * n + i);
+            xv[b] = j >= 0 && j < n ? __ldg(x + j) : T(0);
+        }
+        const T r = MODE != 0 ? rhs[i] : T(0), d = MODE == 2 ? dinv[i] : T(0);
+        T s = M::mul(a[4], xv[4]);
+#pragma unroll
+        for (int b = 0; b < 9; ++b)
+        {
+            const int64_t j = i + off[b];
+            if (b == 4 || j < 0 || j >= n) continue;
+            s = M::add(s, M::mul(a[b], xv[b]));
         }
         if (MODE == 0) y[i] = s;
-        else if (MODE == 1) y[i] = M::sub(rhs[i], s);
-        else y[i] = M::add(x[i], M::mul(M::sub(rhs[i], s), dinv[i]));
+        else if (MODE == 1) y[i] = M::sub(r, s);
+        else y[i] = M::add(xv[4], M::mul(M::sub(r, s), d));
     }
 
     template <typename T>
@@ -160,7 +175,7 @@ namespace hb2
     {
         const int64_t n = (int64_t)A->n, m = (int64_t)A->m;
         const T * b = (const T *)A->bands;
-        if (((uintptr_t)x % 16) == 0)
+        if (((uintptr_t)x % 16) == 0 && A->n > kQ1GatherRows)
         {
             const unsigned grid = ceil_div(A->n, kQ1Threads * RowsPerThread<T>::value);
             q1_kernel<T, MODE><<<grid, kQ1Threads, 0, stream>>>(b, (const T *)x, (T *)y, (const T *)rhs,
