@@ -23,8 +23,8 @@
 //     warp, never the order inside a row.
 //   * longer rows: chunks of W entries ("items") in a compact entry array,
 //     run by warps that stage a chunk's (value, x[column]) pairs in shared
-//     memory with cp.async while lane 0 runs the chain over the previous chunk
-//     (two buffers); a row's chunks stay in one warp.
+//     memory with cp.async while lane 0 runs the chain over an earlier chunk
+//     (eight buffers, or two where long rows are many); a row's chunks stay in one warp.
 // One launch: the CTAs of the long rows first (their chains are the longest),
 // then the slices.  The reference arrays are kept on the host for export.
 #include "hb2_common.cuh"
@@ -87,7 +87,8 @@ namespace
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
     }
     __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-    __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+    template <int N>
+    __device__ __forceinline__ void cp_async_wait_pending() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
     // one slice: lane = row, slots streamed U at a time (columns and values of
     // U slots in flight, then their x entries), the chain in order
@@ -131,71 +132,113 @@ namespace
         else y[row] = s;
     }
 
-    // the long rows of one warp: items k0 .. k1-1, staged two buffers deep
-    template <typename T, bool DEFECT>
+    // the long rows of one warp: items k0 .. k1-1, staged S buffers deep.  The chain over one
+    // chunk (128 dependent fma: 0.3 us in FP32, 0.6 in FP64) is shorter than the two loads
+    // behind a chunk -- columns, then the x they name -- so the columns of the chunk after the
+    // staged ones wait in registers and S - 1 chunks are in flight under the chain.  With one
+    // chunk ahead and its columns fetched on the spot, a row of 2,000 entries took about 20 us,
+    // longer than the rest of a 7-million-entry product.
+    template <typename T, bool DEFECT, int S>
     __device__ __forceinline__ void run_long(uint32_t k0, uint32_t k1, uint32_t lane, T (*buf)[2][kW],
                                              const uint4 * __restrict__ items, const int32_t * __restrict__ lcol,
                                              const T * __restrict__ lval, const T * __restrict__ x,
                                              const T * __restrict__ rhs, T * __restrict__ y)
     {
         if (k0 >= k1) return;
-        auto stage = [&](const uint4 & it, T (*b)[kW]) {
-            const uint32_t n = it.w - it.z;
-            int32_t c[kW / 32];
+        constexpr int E = (int)(kW / 32);
+        uint4 nx = make_uint4(0, 0, 0, 0);     // the next chunk to stage and its columns
+        int32_t c[E];
+        auto columns = [&](uint32_t k) {
+            nx = k < k1 ? __ldg(items + k) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int u = 0; u < (int)(kW / 32); ++u)
+            for (int u = 0; u < E; ++u)
             {
                 const uint32_t i = lane + 32 * u;
-                c[u] = i < n ? __ldg(lcol + it.z + i) : -1;
+                c[u] = i < nx.w - nx.z ? __ldg(lcol + nx.z + i) : -1;
             }
+        };
+        auto stage = [&](T (*b)[kW]) {
 #pragma unroll
-            for (int u = 0; u < (int)(kW / 32); ++u)
+            for (int u = 0; u < E; ++u)
             {
                 const uint32_t i = lane + 32 * u;
-                if (i < n)
+                if (i < nx.w - nx.z)
                 {
-                    cp_async<sizeof(T)>(&b[0][i], lval + it.z + i);
+                    cp_async<sizeof(T)>(&b[0][i], lval + nx.z + i);
                     cp_async<sizeof(T)>(&b[1][i], x + c[u]);
                 }
             }
             cp_async_commit();
         };
+        {
+            // the first chunks: all their columns in flight, then their values and x
+            uint4 n0[S - 1];
+            int32_t c0[S - 1][E];
+#pragma unroll
+            for (int q = 0; q < S - 1; ++q)
+            {
+                columns(k0 + q);
+                n0[q] = nx;
+#pragma unroll
+                for (int u = 0; u < E; ++u) c0[q][u] = c[u];
+            }
+#pragma unroll
+            for (int q = 0; q < S - 1; ++q)
+            {
+                nx = n0[q];
+#pragma unroll
+                for (int u = 0; u < E; ++u) c[u] = c0[q][u];
+                stage(buf[q]);
+            }
+        }
+        columns(k0 + S - 1);
         uint4 cur = __ldg(items + k0);
-        stage(cur, buf[0]);
         T s = T(0);
+        uint32_t bsel = 0, bnew = S - 1;
         for (uint32_t k = k0; k < k1; ++k)
         {
-            const uint32_t bsel = (k - k0) & 1;
-            uint4 nxt = cur;
-            if (k + 1 < k1) nxt = __ldg(items + k + 1);
-            cp_async_wait_all();
-            __syncwarp();
+            cp_async_wait_pending<S - 2>();
+            __syncwarp();              // chunk k is here, and every lane is done with buffer bnew
+            stage(buf[bnew]);
+            columns(k + S);
+            const uint4 it = cur;
+            if (k + 1 < k1) cur = __ldg(items + k + 1);
             if (lane == 0)
             {
-                if (cur.x & kFirstFlag) s = T(0);
-                const uint32_t n = cur.w - cur.z;
+                if (it.x & kFirstFlag) s = T(0);
+                const uint32_t n = it.w - it.z;
                 const T * a = buf[bsel][0];
                 const T * xv = buf[bsel][1];
-                for (uint32_t i = 0; i < n; ++i) s = Arith<T>::fma(a[i], xv[i], s);
-                if (cur.x & kLastFlag)
+                uint32_t i = 0;
+                for (; i + 16 <= n; i += 16)
                 {
-                    const uint32_t row = cur.x & kRowMask;
+                    T av[16], xw[16];
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                    {
+                        av[q] = a[i + q];
+                        xw[q] = xv[i + q];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) s = Arith<T>::fma(av[q], xw[q], s);
+                }
+                for (; i < n; ++i) s = Arith<T>::fma(a[i], xv[i], s);
+                if (it.x & kLastFlag)
+                {
+                    const uint32_t row = it.x & kRowMask;
                     if (DEFECT) y[row] = Arith<T>::sub(__ldg(rhs + row), s);
                     else y[row] = s;
                 }
             }
-            __syncwarp();
-            if (k + 1 < k1)
-            {
-                stage(nxt, buf[bsel ^ 1]);
-                cur = nxt;
-            }
+            bsel = bsel + 1 == S ? 0 : bsel + 1;
+            bnew = bnew + 1 == S ? 0 : bnew + 1;
         }
+        cp_async_wait_pending<0>();
     }
 
     template <typename T, bool DEFECT, int U>
     __global__ void __launch_bounds__(32 * kCsrWarps) csr_kernel(
-        uint32_t long_ctas, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
+        uint32_t long_ctas, int deep, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
         uint32_t nlong_warps, const int32_t * __restrict__ lcol, const T * __restrict__ lval,
         const uint2 * __restrict__ slices, uint32_t nslices, const uint32_t * __restrict__ perm,
         const int32_t * __restrict__ scol, const T * __restrict__ sval, const T * __restrict__ x,
@@ -205,9 +248,17 @@ namespace
         const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (blockIdx.x < long_ctas)
         {
+            if (deep)
+            {
+                // one warp per CTA with all four warps' buffers
+                if (warp == 0)
+                    run_long<T, DEFECT, 2 * kCsrWarps>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), lane, &sbuf[0][0],
+                                                       items, lcol, lval, x, rhs, y);
+                return;
+            }
             const uint32_t w = blockIdx.x * kCsrWarps + warp;
             if (w < nlong_warps)
-                run_long<T, DEFECT>(__ldg(tasks + w), __ldg(tasks + w + 1), lane, sbuf[warp], items, lcol, lval, x,
+                run_long<T, DEFECT, 2>(__ldg(tasks + w), __ldg(tasks + w + 1), lane, sbuf[warp], items, lcol, lval, x,
                                     rhs, y);
             return;
         }
@@ -233,12 +284,15 @@ namespace
     template <typename T, bool DEFECT>
     int launch(hb2_csr A, const void * rhs, const void * x, void * y, cudaStream_t stream)
     {
-        const uint32_t long_ctas = (A->nlong_warps + kCsrWarps - 1) / kCsrWarps;
+        // few long rows: each warp alone in its CTA, eight chunks deep (the same shared memory);
+        // with more of them than SMs the four-warp form keeps more chains resident
+        const int deep = A->nlong_warps <= (uint32_t)num_sms();
+        const uint32_t long_ctas = deep ? A->nlong_warps : (A->nlong_warps + kCsrWarps - 1) / kCsrWarps;
         const uint32_t slice_ctas = (A->nslices + kCsrWarps - 1) / kCsrWarps;
         if (long_ctas + slice_ctas == 0) return HB2_OK;
         auto k = A->unroll == 16 ? csr_kernel<T, DEFECT, 16> : csr_kernel<T, DEFECT, 8>;
         k<<<long_ctas + slice_ctas, 32 * kCsrWarps, 0, stream>>>(
-            long_ctas, A->items, A->tasks, A->nlong_warps, A->lcol, (const T *)A->lval, A->slices, A->nslices,
+            long_ctas, deep, A->items, A->tasks, A->nlong_warps, A->lcol, (const T *)A->lval, A->slices, A->nslices,
             A->perm, A->scol, (const T *)A->sval, (const T *)x, (const T *)rhs, (T *)y);
         count_launches(1);
         HB2_LAUNCH_CHECK("csr_kernel");
