@@ -338,6 +338,8 @@ namespace hb2
             if (red && ! ws) return fail(HB2_ERR_ARG, "fused reduction without a workspace");
             return launch_q1_single(A, mode, x, y, aux, red, want_sqrt, ws, stream);
         }
+        if (b.nvec == 1 && ! b.list && ! b.active && grid9_applies(A, mode, red != 0))
+            return launch_grid9(A, mode, x, y, aux, aux2, red, want_sqrt, ws, stream, flags);
         // the launch shape: the class's tuned one, except where a Q1 gather layout
         // hands this launch to the general row-pattern kernel (256 threads)
         const int cls = red != 0;

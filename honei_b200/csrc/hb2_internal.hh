@@ -140,6 +140,8 @@ struct hb2_ell_s
     uint32_t q1g_m = 0;
     double q1g_v[9] = {};
     double q1g_vb = 0;
+    // points per line when the rows have that structure with other values (ell_grid9.cu), else 0
+    uint32_t g9_m = 0;
 
     template <typename T> hb2::EllView<T> view() const
     {
@@ -336,6 +338,10 @@ namespace hb2
         uint32_t nvec = 1, max_vec = 1;
         uint64_t vstride = 0, cstride = 0, cap = 0;
     };
+    // nine-point grid matrices with any values, on the plain arrays without the columns (ell_grid9.cu)
+    bool grid9_applies(const hb2_ell_s * A, int mode, bool reducing);
+    int launch_grid9(const hb2_ell_s * A, int mode, const void * x, void * y, const void * aux, const void * aux2,
+                     double * red, int want_sqrt, const Workspace * ws, cudaStream_t stream, int flags);
     bool q1_transfer_kernels_enabled();   // HB2_Q1_TRANSFER=0 turns them off (ell.cu)
     int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream);
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);

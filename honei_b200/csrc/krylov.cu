@@ -170,7 +170,7 @@ namespace
     struct LoopArgs
     {
         EllView<double> A;
-        uint32_t m;                     // Q1 grid operator (q1g_m): its rows from the grid
+        uint32_t m;                     // Q1 grid operator (q1g_m) or nine-point grid matrix (g9_m)
         double a[9], ab;
         uint32_t n, rows;               // rows per thread
         uint64_t max_iters;
@@ -216,17 +216,20 @@ namespace
         return *ok != 0;
     }
 
-    // KT: 9 slots unrolled, 0 any number, -1 the Q1 grid
+    // KT: 9 slots unrolled, 0 any number, -1 the Q1 grid, -2 a nine-point grid matrix's values
     template <int KT>
     __device__ __forceinline__ double loop_row(const LoopArgs & g, uint32_t row, const double * p)
     {
         double s = 0.0;
-        if constexpr (KT == -1)
+        if constexpr (KT < 0)
         {
             const uint32_t m = g.m, i = row / m, j = row - i * m;
-            if (i == 0 || j == 0 || i == m - 1 || j == m - 1) return __dadd_rn(0.0, __dmul_rn(g.ab, p[row]));
+            if (i == 0 || j == 0 || i == m - 1 || j == m - 1)
+                return __dadd_rn(0.0, __dmul_rn(KT == -1 ? g.ab : __ldg(g.A.val + row), p[row]));
             const double * c = p + row;
-            double xv[9];
+            double xv[9], a[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) a[q] = KT == -1 ? g.a[q] : __ldg(g.A.val + (uint64_t)q * g.A.ld + row);
 #pragma unroll
             for (int q = 0; q < 3; ++q)
             {
@@ -235,7 +238,7 @@ namespace
                 xv[6 + q] = c[(int)m + (q - 1)];
             }
 #pragma unroll
-            for (int q = 0; q < 9; ++q) s = __dadd_rn(s, __dmul_rn(g.a[q], xv[q]));
+            for (int q = 0; q < 9; ++q) s = __dadd_rn(s, __dmul_rn(a[q], xv[q]));
         }
         else if constexpr (KT > 0)
         {
@@ -741,7 +744,7 @@ namespace
     {
         LoopArgs g = {};
         g.A = K->A->view<double>();
-        g.m = K->A->q1g_m;
+        g.m = K->A->q1g_m ? K->A->q1g_m : K->A->g9_m;
         for (int k = 0; k < 9; ++k) g.a[k] = K->A->q1g_v[k];
         g.ab = K->A->q1g_vb;
         g.n = (uint32_t)K->n;
@@ -758,7 +761,9 @@ namespace
         g.arrived = K->ws->bar_words;
         g.error = K->ws->error;
         k_cg_loop_init<<<1, 1, 0, s>>>(K->st, g.arrived, g.error);
-        const cudaError_t e = g.m ? launch_loop<-1>(g, s) : K->A->K == 9 ? launch_loop<9>(g, s) : launch_loop<0>(g, s);
+        const cudaError_t e = K->A->q1g_m   ? launch_loop<-1>(g, s)
+                              : K->A->g9_m  ? launch_loop<-2>(g, s)
+                              : K->A->K == 9 ? launch_loop<9>(g, s) : launch_loop<0>(g, s);
         count_launches(2);
         if (e != cudaSuccess) return cuda_status(e, "krylov CG loop");
         HB2_LAUNCH_CHECK("krylov CG loop");

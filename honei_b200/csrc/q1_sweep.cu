@@ -9,25 +9,36 @@ namespace hb2
     int q1_sweep_f32(const Q1SweepArgs<float> & g, bool wide, bool uni, int S, int head, int tail, bool pvec,
                      const SweepLaunch & l);
 
-    // every row against the two rows of a Q1 grid operator: interior rows hold the nine
-    // couplings of v in ascending column order, boundary rows one diagonal entry vb in slot 0
+    // every row against the two kinds of rows of a Q1 grid operator: interior rows nine columns
+    // in ascending order, boundary rows one diagonal entry in slot 0 (bad bit 0: another
+    // structure); all interior rows with the values ref[0 .. 8], all boundary rows with ref[9]
+    // (bit 1: other values)
     template <typename T>
     __global__ void q1_grid_check_kernel(EllView<T> A, uint32_t m, const T * __restrict__ ref, int * bad)
     {
         const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (r >= A.rows) return;
-        const uint32_t i = (uint32_t)(r / m), j = (uint32_t)(r - (uint64_t)i * m);
+        const uint32_t i = (uint32_t)r / m, j = (uint32_t)r - i * m;
         const bool bnd = i == 0 || j == 0 || i == m - 1 || j == m - 1;
-        bool ok = true;
+        bool shape = true, same = true;
 #pragma unroll
         for (int k = 0; k < 9; ++k)
         {
             const int32_t c = A.col[k * A.ld + r];
             const T v = A.val[k * A.ld + r];
-            if (bnd) ok = ok && (k == 0 ? (c == (int32_t)r && v == ref[9]) : c < 0);
-            else ok = ok && c == (int32_t)((int64_t)r + (k / 3 - 1) * (int64_t)m + (k % 3 - 1)) && v == ref[k];
+            if (bnd)
+            {
+                shape = shape && (k == 0 ? c == (int32_t)r : c < 0);
+                if (k == 0) same = same && v == ref[9];
+            }
+            else
+            {
+                shape = shape && c == (int32_t)((int64_t)r + (k / 3 - 1) * (int64_t)m + (k % 3 - 1));
+                same = same && v == ref[k];
+            }
         }
-        if (! ok) *bad = 1;
+        if (! shape) atomicOr(bad, 1);
+        if (! same) atomicOr(bad, 2);
     }
 
     template <typename T>
@@ -52,6 +63,7 @@ namespace hb2
         HB2_CUDA(cudaMemcpyAsync(ref, dref, sizeof(ref), cudaMemcpyDeviceToHost, stream));
         HB2_CUDA(cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, stream));
         HB2_CUDA(cudaStreamSynchronize(stream));
+        if (bad == 2) A->g9_m = m;
         if (bad) return HB2_OK;
         for (int k = 0; k < 9; ++k) A->q1g_v[k] = (double)ref[k];
         A->q1g_vb = (double)ref[9];
@@ -61,7 +73,7 @@ namespace hb2
 
     int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream)
     {
-        A->q1g_m = 0;
+        A->q1g_m = A->g9_m = 0;
         if (A->rows != A->cols || A->K != 9 || A->rows < 9 || A->rows >= (1ull << 31)) return HB2_OK;
         uint64_t m = 3;
         while (m * m < A->rows) ++m;
