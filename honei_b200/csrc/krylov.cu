@@ -189,8 +189,9 @@ namespace
     {
         if (threadIdx.x == 0)
         {
-            __threadfence();
-            atomicAdd(g.arrived, 1u);
+            // the release covers the block's writes before the caller's block barrier, the acquire
+            // its reads after the one below (a full fence each side cost the round trips twice)
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.arrived) : "memory");
             *ok = 1;
             unsigned long long t0 = 0;
             for (unsigned spin = 0;; ++spin)
@@ -210,7 +211,6 @@ namespace
                     }
                 }
             }
-            __threadfence();
         }
         __syncthreads();
         return *ok != 0;
