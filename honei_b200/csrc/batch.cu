@@ -54,10 +54,10 @@ namespace hb2
 
     constexpr int kMaxGroups = 14;
     constexpr int kOuterThreads = 256;
-    // rows per thread and work item, interleaved over the block.  Four instead of two halves
-    // the reductions (a block sum, a fence and two tickets an item); measured with the stencil
-    // product below on the 128-system batch, see hb2_batch_s.
-    constexpr int kOuterRows = 4;
+    // rows per thread and work item, interleaved over the block: an item ends with a block sum,
+    // a fence and two tickets, so fewer and larger items (128-system batch, a step's outer
+    // kernels with 4 rows: 143 / 187 / 93 / 60 us where their bytes need 50 / 185 / 36 / 60)
+    constexpr int kOuterRows = 8;
 
     constexpr int kMaxLevels = 16;
 
@@ -133,20 +133,22 @@ namespace hb2
         double acc = 0.0;
         if (G.m)
         {
+            // a boundary row reads its own value nine times and keeps the one product
             const uint32_t m = G.m, r = (uint32_t)row, i = r / m, j = r - i * m;
-            if (i == 0 || j == 0 || i == m - 1 || j == m - 1) return __dadd_rn(0.0, __dmul_rn(G.ab, __ldg(x + row)));
+            const bool edge = i == 0 || j == 0 || i == m - 1 || j == m - 1;
+            const int dm = edge ? 0 : (int)m, d1 = edge ? 0 : 1;
             const double * c = x + row;
             double xv[9];
 #pragma unroll
             for (int q = 0; q < 3; ++q)
             {
-                xv[q] = __ldg(c - (int)m + (q - 1));
-                xv[3 + q] = __ldg(c + (q - 1));
-                xv[6 + q] = __ldg(c + (int)m + (q - 1));
+                xv[q] = __ldg(c - dm + (q - 1) * d1);
+                xv[3 + q] = __ldg(c + (q - 1) * d1);
+                xv[6 + q] = __ldg(c + dm + (q - 1) * d1);
             }
 #pragma unroll
             for (int q = 0; q < 9; ++q) acc = __dadd_rn(acc, __dmul_rn(G.a[q], xv[q]));
-            return acc;
+            return edge ? __dadd_rn(0.0, __dmul_rn(G.ab, xv[4])) : acc;
         }
         for (uint32_t k = 0; k < G.A.K; ++k)
         {
@@ -194,22 +196,26 @@ namespace hb2
     // Phase A.  kNew: r = b - A x (math/cg.hh:161), ||r||^2; kRun: v = A p,
     // v.p (cg.hh:174-175).  Either way the inner rhs of the finest level gets
     // (float) r and the inner correction 0, ready for the preconditioner.
-    __global__ void __launch_bounds__(kOuterThreads) bpcg_phase_a_kernel(const __grid_constant__ OuterPlan P, SlotScalars S)
+    __global__ void __launch_bounds__(kOuterThreads, 6) bpcg_phase_a_kernel(const __grid_constant__ OuterPlan P, SlotScalars S)
     {
         walk(P, S.live, S.plan->live_start, S.plan->live_item0, [&](const OuterGroup & G, uint32_t j, uint32_t lj, uint32_t blk) {
             const bool init = S.state[j] == kNew;
             const uint64_t o = (uint64_t)lj * G.vs, o32 = (uint64_t)j * G.vs32;
             const double * xp = (init ? G.x : G.p) + o;
             double part = 0.0;
-#pragma unroll
+            // rows past the end compute the last one again, unconditionally: the loads of several
+            // rows are in flight together
+#pragma unroll 2
             for (int i = 0; i < kOuterRows; ++i)
             {
-                const uint64_t row = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
-                if (row >= G.n) break;
-                const double acc = row_product(G, row, xp);
+                const uint64_t at = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
+                const uint64_t row = min(at, G.n - 1);
+                const double acc = row_product(G, row, xp), xc = xp[row];
+                const double bv = init ? G.b[o + row] : 0.0;
+                if (at >= G.n) continue;
                 if (init)
                 {
-                    const double d = __dsub_rn(G.b[o + row], acc);
+                    const double d = __dsub_rn(bv, acc);
                     G.r[o + row] = d;
                     G.b32[o32 + row] = __double2float_rn(d);
                     if (G.clear32) G.x32[o32 + row] = 0.f;
@@ -218,7 +224,7 @@ namespace hb2
                 else
                 {
                     G.v[o + row] = acc;
-                    part = fma(acc, xp[row], part);
+                    part = fma(acc, xc, part);
                 }
             }
             finish(G, lj, blk, part, S.red_a + j, [] {});
@@ -391,9 +397,10 @@ namespace hb2
 #pragma unroll
             for (int i = 0; i < kOuterRows; ++i)
             {
-                const uint64_t row = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
-                if (row >= G.n) break;
-                part = fma(G.r[o + row], (double)G.x32[o32 + row], part);
+                const uint64_t at = (uint64_t)blk * (kOuterThreads * kOuterRows) + i * kOuterThreads + threadIdx.x;
+                const uint64_t row = min(at, G.n - 1);
+                const double r = G.r[o + row], z = (double)G.x32[o32 + row];
+                if (at < G.n) part = fma(r, z, part);
             }
             finish(G, lj, blk, part, S.red_z + j, [&] {
                 const double an_new = S.red_z[j];

@@ -186,6 +186,7 @@ namespace hb2
             pr[j] = rr[j];
             if (row < n) sp[row] = pr[j];
         }
+        if (exact != kCgExact && lane == 0) sp[n] = sp2[n] = T(0);     // (the exact mode's dots use this memory)
         __syncwarp();
         const T eps = T(eps_d);
         T alpha = dot(rr, rr);
@@ -202,8 +203,6 @@ namespace hb2
             //   x += a p; r -= a s; w = A r; g = (r, r); d = (w, r);
             //   b = g / g_old; a = g / (d - b g / a_old); p = r + b p; s = w + b s
             T sr[RPL], wr[RPL];
-            if (lane == 0) sp[n] = sp2[n] = T(0);
-            __syncwarp();
             spmv_tree(wr, sp);   // w0 = A r0 (sp holds r0 = p0)
             T gam = alpha, del;
             {
@@ -274,9 +273,17 @@ namespace hb2
         }
         while (it < max_iters)
         {
-            spmv(vr);
+            // the tree-ordered mode takes the fused product and reciprocals, that of the old
+            // alpha while the product's dot is on its way
+            T inv_alpha = T(0);
+            if (exact == kCgExact) spmv(vr);
+            else
+            {
+                spmv_tree(vr, sp);
+                inv_alpha = Recip<T>::rn(guard(alpha));
+            }
             const T temp = dot(vr, pr);
-            const T lambda = M::div(alpha, guard(temp));
+            const T lambda = exact == kCgExact ? M::div(alpha, guard(temp)) : M::mul(alpha, Recip<T>::rn(guard(temp)));
             const T mlambda = -lambda;
 #pragma unroll
             for (int j = 0; j < RPL; ++j)
@@ -286,7 +293,7 @@ namespace hb2
             }
             const T alpha_old = alpha;
             alpha = dot(rr, rr);
-            const T talpha = M::div(alpha, guard(alpha_old));
+            const T talpha = exact == kCgExact ? M::div(alpha, guard(alpha_old)) : M::mul(alpha, inv_alpha);
             __syncwarp();   // every lane is done gathering the old p
 #pragma unroll
             for (int j = 0; j < RPL; ++j)
