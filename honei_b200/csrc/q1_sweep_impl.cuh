@@ -56,17 +56,19 @@ namespace hb2
 #undef HB2_SG
     }
 
-    // CW columns a lane when wide, else CN (equal: one form); the general nine-value form
-    // and the given Jacobi vector (pvec) run wide only
+    // CW columns a lane when wide, else CN; the general nine-value form in one width
     template <typename T, int CW, int CN>
     static int q1_sweep_typed(const Q1SweepArgs<T> & g, bool wide, bool uni, int S, int head, int tail, bool pvec,
                               const SweepLaunch & l)
     {
-        if (sweep_single(tail)) return uni ? q1_single<T, CW, true>(g, tail, l) : q1_single<T, CW, false>(g, tail, l);
+        // the passes without sweeps and the given Jacobi vector: the form that is fast on the
+        // middle grids too (16 bytes a lane in FP64, 8 in FP32)
+        constexpr int CM = sizeof(T) == 8 ? CW : CN;
+        if (sweep_single(tail)) return uni ? q1_single<T, CM, true>(g, tail, l) : q1_single<T, CM, false>(g, tail, l);
         if (pvec)
-            return uni ? q1_sweep_s<T, CW, true, kSweepLoad, kSweepStore, true>(g, S, l)
-                       : q1_sweep_s<T, CW, false, kSweepLoad, kSweepStore, true>(g, S, l);
-        if (! uni) return q1_sweep_kind<T, CW, false>(g, S, head, tail, l);
+            return uni ? q1_sweep_s<T, CM, true, kSweepLoad, kSweepStore, true>(g, S, l)
+                       : q1_sweep_s<T, CM, false, kSweepLoad, kSweepStore, true>(g, S, l);
+        if (! uni) return q1_sweep_kind<T, CM, false>(g, S, head, tail, l);
         return wide ? q1_sweep_kind<T, CW, true>(g, S, head, tail, l) : q1_sweep_kind<T, CN, true>(g, S, head, tail, l);
     }
 }
