@@ -11,9 +11,10 @@
 //   coarser levels: x = dinv (.) rhs, n_pre - 1 sweeps on A x = rhs;
 //   then d = rhs - A x and rhs(coarser) = R d (matrix-free, Dirichlet mask);
 //   coarsest level: the banded ConjugateGradients (math/conjugate_gradients.hh:491-560)
-//     in one thread -- its dot products in the reference's sequential order;
+//     in one warp or thread -- its dot products in the reference's sequential order;
 //   upwards: c = P x(coarser), x += alpha c, n_pre Jacobi sweeps (the reference's
-//     kernel uses n_pre_smooth for the post-smoothing too), d = rhs - A x.
+//     kernel uses n_pre_smooth for the post-smoothing too), on the finest level d = rhs - A x.
+// The small levels below the finest run in one block (k_lmg_bottom).
 // A Jacobi sweep is one fused banded kernel y = x + (rhs - A x) (.) dinv with the
 // reference's rounding; every kernel but the finest norm is bit-identical to the
 // reference, and the norm (a tree reduction) only decides when to stop.

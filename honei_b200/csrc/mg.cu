@@ -11,6 +11,10 @@
 //   Prolongation + Sum                                  -> one SpMV-add pass
 //   coarsest CGSolver                                   -> one thread block, shared memory
 //   convergence Defect + Norm                           -> one pass
+// On Q1 grid hierarchies a level takes two passes a cycle instead (q1_sweep.cuh): all
+// pre-smoothing sweeps with the defect and its restriction, the prolongation with all
+// post-smoothing sweeps (and the convergence norm); the smallest levels and the coarsest
+// CG run in one block (q1_bottom.cu).
 // and the MGSolver loop itself runs on the device: the solve graph is the
 // initial defect, a conditional WHILE node whose body is one V-cycle plus the
 // convergence defect and a one-thread decision kernel, and the copy of the

@@ -1,6 +1,7 @@
 // BandedMatrixQx<Q1Type, DT> SpMV and defect (la/product.hh:370-403,
-// math/defect.hh:194-198) with the x row-windows staged in shared memory by
-// TMA bulk copies (cp.async.bulk, no multicast, completion on an mbarrier).
+// math/defect.hh:194-198): with the x row-windows staged in shared memory by
+// TMA bulk copies (cp.async.bulk, no multicast, completion on an mbarrier), on
+// small grids by plain loads (q1_kernel_direct).
 //
 // A block owns B consecutive rows [r0, r0+B).  The nine bands touch three
 // windows of x: [r0-m-1, r0+B-m+1), [r0-1, r0+B+1), [r0+m-1, r0+B+m+1).  Each is
