@@ -48,6 +48,9 @@ namespace
     constexpr uint32_t kLastFlag = 0x40000000u;          // last chunk: the sum is stored
     constexpr uint32_t kRowMask = 0x3fffffffu;
     constexpr uint64_t kMaxBlockSize = 1024;
+    constexpr uint32_t kWinBytes = 64 * 1024;            // largest staged window of x
+    constexpr uint32_t kWinWarps = kSigma / 32;          // one slice a warp, one window a CTA
+    constexpr uint32_t kNoWindow = 0xffffffffu;          // a window's span does not fit
 }
 
 struct hb2_csr_s
@@ -67,6 +70,11 @@ struct hb2_csr_s
     uint32_t nslices = 0;
     uint64_t nslots = 0;
     int unroll = 8;                // slots per lane and round (8 or 16)
+    // x windows: [first column, columns) of each window of kSigma short rows; the largest
+    // one's size in bytes; staged: the kernel that copies them to shared memory runs
+    uint2 * xwin = nullptr;
+    uint32_t nwindows = 0, win_bytes = 0;
+    bool staged = false;
     // long rows
     uint4 * items = nullptr;       // (row | flags, 0, first entry, end entry)
     uint32_t * tasks = nullptr;    // nlong_warps + 1 item offsets
@@ -132,12 +140,8 @@ namespace
         else y[row] = s;
     }
 
-    // the long rows of one warp: items k0 .. k1-1, staged S buffers deep.  The chain over one
-    // chunk (128 dependent fma: 0.3 us in FP32, 0.6 in FP64) is shorter than the two loads
-    // behind a chunk -- columns, then the x they name -- so the columns of the chunk after the
-    // staged ones wait in registers and S - 1 chunks are in flight under the chain.  With one
-    // chunk ahead and its columns fetched on the spot, a row of 2,000 entries took about 20 us,
-    // longer than the rest of a 7-million-entry product.
+    // the long rows of one warp where long rows are many: items k0 .. k1-1, staged S buffers deep,
+    // the next chunk's columns in registers
     template <typename T, bool DEFECT, int S>
     __device__ __forceinline__ void run_long(uint32_t k0, uint32_t k1, uint32_t lane, T (*buf)[2][kW],
                                              const uint4 * __restrict__ items, const int32_t * __restrict__ lcol,
@@ -236,6 +240,129 @@ namespace
         cp_async_wait_pending<0>();
     }
 
+    // The long rows of one warp alone in its CTA.  The chain over a chunk (128 dependent fma, 0.3
+    // us in FP32) is far shorter than what stands behind a chunk -- its item, its columns, the x
+    // they name, each a load that needs the one before -- so all three run ahead of it: items by
+    // the warp's lanes (32 at a time), columns by cp.async kDeepL chunks before they are used,
+    // values and x by cp.async kDeepS - 1 chunks before the chain.  A 2,000-entry FP32 row took
+    // 27 us with one chunk ahead and 16 us with seven but their columns fetched one step ahead.
+    constexpr int kDeepS = 8, kDeepL = 7, kDeepC = 16;
+    template <typename T> constexpr size_t deep_bytes() { return kDeepS * 2 * kW * sizeof(T) + kDeepC * kW * sizeof(int32_t); }
+
+    template <typename T, bool DEFECT>
+    __device__ __forceinline__ void run_long_deep(uint32_t k0, uint32_t k1, uint32_t lane, unsigned char * smem,
+                                                  const uint4 * __restrict__ items, const int32_t * __restrict__ lcol,
+                                                  const T * __restrict__ lval, const T * __restrict__ x,
+                                                  const T * __restrict__ rhs, T * __restrict__ y)
+    {
+        if (k0 >= k1) return;
+        T (*buf)[2][kW] = reinterpret_cast<T (*)[2][kW]>(smem);
+        int32_t (*cb)[kW] = reinterpret_cast<int32_t (*)[kW]>(smem + kDeepS * 2 * kW * sizeof(T));
+        constexpr int E = (int)(kW / 32);
+        const uint4 none = make_uint4(0, 0, 0, 0);
+        uint32_t kb = k0;                      // items kb .. kb + 63, one and one a lane
+        uint4 i0 = k0 + lane < k1 ? __ldg(items + k0 + lane) : none;
+        uint4 i1 = k0 + 32 + lane < k1 ? __ldg(items + k0 + 32 + lane) : none;
+        auto item = [&](uint32_t k) -> uint4 {
+            const uint4 & v = k - kb < 32 ? i0 : i1;
+            const int l = (int)((k - kb) & 31);
+            return make_uint4(__shfl_sync(0xffffffffu, v.x, l), 0, __shfl_sync(0xffffffffu, v.z, l),
+                              __shfl_sync(0xffffffffu, v.w, l));
+        };
+        auto columns = [&](uint32_t k) {
+            const uint4 it = item(k);          // (0, 0) past the last one
+#pragma unroll
+            for (int u = 0; u < E; ++u)
+            {
+                const uint32_t i = lane + 32 * u;
+                if (i < it.w - it.z) cp_async<4>(&cb[k % kDeepC][i], lcol + it.z + i);
+            }
+        };
+        auto stage = [&](uint32_t k) {
+            const uint4 it = item(k);
+#pragma unroll
+            for (int u = 0; u < E; ++u)
+            {
+                const uint32_t i = lane + 32 * u;
+                if (i < it.w - it.z)
+                {
+                    cp_async<sizeof(T)>(&buf[k % kDeepS][0][i], lval + it.z + i);
+                    cp_async<sizeof(T)>(&buf[k % kDeepS][1][i], x + cb[k % kDeepC][i]);   // the lane's own copy
+                }
+            }
+        };
+        for (uint32_t q = 0; q < kDeepS - 1 + kDeepL; ++q) columns(k0 + q);
+        cp_async_commit();
+        cp_async_wait_pending<0>();
+        for (uint32_t q = 0; q < kDeepS - 1; ++q)
+        {
+            stage(k0 + q);
+            cp_async_commit();
+        }
+        T s = T(0);
+        for (uint32_t k = k0; k < k1; ++k)
+        {
+            if (k - kb == 32)
+            {
+                kb += 32;
+                i0 = i1;
+                i1 = kb + 32 + lane < k1 ? __ldg(items + kb + 32 + lane) : none;
+            }
+            cp_async_wait_pending<kDeepS - 2>();
+            __syncwarp();                      // chunk k is here, chunk k - 1 is done with
+            stage(k + kDeepS - 1);
+            columns(k + kDeepS - 1 + kDeepL);
+            cp_async_commit();
+            const uint4 it = item(k);
+            if (lane == 0)
+            {
+                if (it.x & kFirstFlag) s = T(0);
+                const uint32_t n = it.w - it.z;
+                const T * a = buf[k % kDeepS][0];
+                const T * xv = buf[k % kDeepS][1];
+                // 128-bit reads of the next entries under the chain over these
+                constexpr uint32_t V = 16 / sizeof(T), G = 2 * V;
+                union Quad { int4 q[G / V]; T t[G]; };
+                Quad av, xw, an, xn;
+                auto group = [&](uint32_t i, Quad & p, Quad & q) {
+#pragma unroll
+                    for (uint32_t h = 0; h < G / V; ++h)
+                    {
+                        p.q[h] = *reinterpret_cast<const int4 *>(a + i + h * V);
+                        q.q[h] = *reinterpret_cast<const int4 *>(xv + i + h * V);
+                    }
+                };
+                auto chain = [&](const Quad & p, const Quad & q) {
+#pragma unroll
+                    for (uint32_t h = 0; h < G; ++h) s = Arith<T>::fma(p.t[h], q.t[h], s);
+                };
+                // two groups a turn, changing places: no copies (they and a chunk's other
+                // instructions, not the fma latency, set the pace of a single warp)
+                uint32_t i = 0;
+                if (n >= 2 * G)
+                {
+                    group(0, av, xw);
+#pragma unroll 1
+                    for (; i + 2 * G <= n; i += 2 * G)
+                    {
+                        group(i + G, an, xn);
+                        chain(av, xw);
+                        group(i + 4 * G <= n ? i + 2 * G : i, av, xw);
+                        chain(an, xn);
+                    }
+                }
+                for (; i < n; ++i) s = Arith<T>::fma(a[i], xv[i], s);
+                if (it.x & kLastFlag)
+                {
+                    const uint32_t row = it.x & kRowMask;
+                    if (DEFECT) y[row] = Arith<T>::sub(__ldg(rhs + row), s);
+                    else y[row] = s;
+                }
+            }
+        }
+        cp_async_wait_pending<0>();
+    }
+
     template <typename T, bool DEFECT, int U>
     __global__ void __launch_bounds__(32 * kCsrWarps) csr_kernel(
         uint32_t long_ctas, int deep, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
@@ -244,26 +371,103 @@ namespace
         const int32_t * __restrict__ scol, const T * __restrict__ sval, const T * __restrict__ x,
         const T * __restrict__ rhs, T * __restrict__ y)
     {
-        __shared__ __align__(16) T sbuf[kCsrWarps][2][2][kW];     // [warp][buffer][value | x][i]
+        // the long rows' buffers: [warp][buffer][value | x][i], or those of one warp (run_long_deep)
+        constexpr size_t kBytes = kCsrWarps * 2 * 2 * kW * sizeof(T);
+        __shared__ __align__(16) unsigned char sbuf[deep_bytes<T>() > kBytes ? deep_bytes<T>() : kBytes];
         const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (blockIdx.x < long_ctas)
         {
             if (deep)
             {
-                // one warp per CTA with all four warps' buffers
                 if (warp == 0)
-                    run_long<T, DEFECT, 2 * kCsrWarps>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), lane, &sbuf[0][0],
-                                                       items, lcol, lval, x, rhs, y);
+                    run_long_deep<T, DEFECT>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), lane, sbuf, items, lcol,
+                                             lval, x, rhs, y);
                 return;
             }
             const uint32_t w = blockIdx.x * kCsrWarps + warp;
             if (w < nlong_warps)
-                run_long<T, DEFECT, 2>(__ldg(tasks + w), __ldg(tasks + w + 1), lane, sbuf[warp], items, lcol, lval, x,
+                run_long<T, DEFECT, 2>(__ldg(tasks + w), __ldg(tasks + w + 1), lane,
+                                       reinterpret_cast<T (*)[2][kW]>(sbuf) + 2 * warp, items, lcol, lval, x,
                                     rhs, y);
             return;
         }
         const uint32_t slice = (blockIdx.x - long_ctas) * kCsrWarps + warp;
         if (slice < nslices) run_slice<T, DEFECT, U>(slice, lane, slices, perm, scol, sval, x, rhs, y);
+    }
+
+    // The slices of one window of kSigma rows per CTA, with the window's span of x in shared
+    // memory.  Gathers whose lanes fall on many cache lines cost the L1 one line each -- about
+    // 28 cycles a warp on random columns near the diagonal, 21 of the 25 us of a product with
+    // 7 million of them -- where shared memory pays bank conflicts only.  The long rows' CTAs
+    // come first, as in csr_kernel, one warp each.
+    template <typename T, bool DEFECT, int U>
+    __global__ void __launch_bounds__(32 * kWinWarps, 2) csr_staged_kernel(
+        uint32_t long_ctas, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
+        const int32_t * __restrict__ lcol, const T * __restrict__ lval, const uint2 * __restrict__ xwin,
+        const uint2 * __restrict__ slices, uint32_t nslices, const uint32_t * __restrict__ perm,
+        const int32_t * __restrict__ scol, const T * __restrict__ sval, const T * __restrict__ x,
+        const T * __restrict__ rhs, T * __restrict__ y)
+    {
+        extern __shared__ __align__(16) unsigned char csr_smem[];
+        const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (blockIdx.x < long_ctas)
+        {
+            __shared__ __align__(16) unsigned char lbuf[deep_bytes<T>()];
+            if (warp == 0)
+                run_long_deep<T, DEFECT>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), lane, lbuf, items, lcol, lval,
+                                         x, rhs, y);
+            return;
+        }
+        T * xs = reinterpret_cast<T *>(csr_smem);
+        const uint32_t w = blockIdx.x - long_ctas, slice = w * kWinWarps + warp;
+        const uint2 win = __ldg(xwin + w);
+        const bool direct = win.y == kNoWindow;      // a window too wide to stage
+        for (uint32_t i = threadIdx.x; ! direct && i < win.y; i += 32 * kWinWarps) cp_async<sizeof(T)>(xs + i, x + win.x + i);
+        cp_async_commit();
+        // the slice's first slots while the window is on its way
+        uint32_t row = 0xffffffffu;
+        uint2 d = make_uint2(0, 0);
+        T rh = T(0);
+        if (slice < nslices)
+        {
+            d = __ldg(slices + slice);
+            row = __ldg(perm + 32 * slice + lane);
+            if (DEFECT && row != 0xffffffffu) rh = __ldg(rhs + row);
+        }
+        const int32_t * cp = scol + d.x + lane;
+        const T * vp = sval + d.x + lane;
+        int32_t c[U];
+        T a[U];
+        auto load = [&](uint32_t k) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                const bool in = k + u < d.y;
+                c[u] = in ? __ldcs(cp + 32 * (k + u)) : -1;
+                a[u] = in ? __ldcs(vp + 32 * (k + u)) : T(0);
+            }
+        };
+        load(0);
+        cp_async_wait_pending<0>();
+        __syncthreads();
+        T s = T(0);
+        for (uint32_t k = 0; k < d.y; k += U)
+        {
+            if (k) load(k);
+            if (direct)
+            {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (c[u] >= 0) s = Arith<T>::fma(a[u], __ldg(x + c[u]), s);
+            }
+            else
+            {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (c[u] >= 0) s = Arith<T>::fma(a[u], xs[(uint32_t)c[u] - win.x], s);
+            }
+        }
+        if (row != 0xffffffffu) y[row] = DEFECT ? Arith<T>::sub(rh, s) : s;
     }
 
     int csr_free(hb2_csr_s * A)
@@ -277,6 +481,7 @@ namespace
         cudaFree(A->tasks);
         cudaFree(A->lcol);
         cudaFree(A->lval);
+        cudaFree(A->xwin);
         delete A;
         return HB2_OK;
     }
@@ -284,12 +489,23 @@ namespace
     template <typename T, bool DEFECT>
     int launch(hb2_csr A, const void * rhs, const void * x, void * y, cudaStream_t stream)
     {
-        // few long rows: each warp alone in its CTA, eight chunks deep (the same shared memory);
+        // few long rows: each warp alone in its CTA, eight chunks deep;
         // with more of them than SMs the four-warp form keeps more chains resident
         const int deep = A->nlong_warps <= (uint32_t)num_sms();
         const uint32_t long_ctas = deep ? A->nlong_warps : (A->nlong_warps + kCsrWarps - 1) / kCsrWarps;
         const uint32_t slice_ctas = (A->nslices + kCsrWarps - 1) / kCsrWarps;
         if (long_ctas + slice_ctas == 0) return HB2_OK;
+        if (A->staged)
+        {
+            auto ks = A->unroll == 16 ? csr_staged_kernel<T, DEFECT, 16> : csr_staged_kernel<T, DEFECT, 8>;
+            HB2_CUDA(cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->win_bytes));
+            ks<<<A->nlong_warps + A->nwindows, 32 * kWinWarps, A->win_bytes, stream>>>(
+                A->nlong_warps, A->items, A->tasks, A->lcol, (const T *)A->lval, A->xwin, A->slices, A->nslices, A->perm,
+                A->scol, (const T *)A->sval, (const T *)x, (const T *)rhs, (T *)y);
+            count_launches(1);
+            HB2_LAUNCH_CHECK("csr_staged_kernel");
+            return HB2_OK;
+        }
         auto k = A->unroll == 16 ? csr_kernel<T, DEFECT, 16> : csr_kernel<T, DEFECT, 8>;
         k<<<long_ctas + slice_ctas, 32 * kCsrWarps, 0, stream>>>(
             long_ctas, deep, A->items, A->tasks, A->nlong_warps, A->lcol, (const T *)A->lval, A->slices, A->nslices,
@@ -299,21 +515,25 @@ namespace
         return HB2_OK;
     }
 
-    // Slots loaded per lane and round in the sliced part: 8 or 16, whichever
-    // runs the product faster on this matrix (timed at creation when it holds
-    // at least 2^20 slots; bit-identical results either way).  Measured on the
+    // Slots loaded per lane and round in the sliced part, 8 or 16, and x gathered from
+    // global memory or staged by window: whichever runs the product fastest on this
+    // matrix (timed at creation when it holds at least 2^18 slots; bit-identical
+    // results either way).  Measured on the
     // level-11 Q1 operator: FP64 108.6 us (16) / 127.0 us (8), FP32 83.9 us (16)
     // / 75.0 us (8).  HB2_CSR_U=8|16 fixes it.
     template <typename T>
     int choose_unroll(hb2_csr_s * A, cudaStream_t stream)
     {
         A->unroll = 8;
+        A->staged = false;
         if (const char * env = getenv("HB2_CSR_U"))
         {
             A->unroll = atoi(env) == 16 ? 16 : 8;
+            const char * st = getenv("HB2_CSR_STAGED");     // with HB2_CSR_U: 1 stages x where it fits
+            A->staged = st && atoi(st) == 1 && A->win_bytes;
             return HB2_OK;
         }
-        if (A->nslots + A->nlong_entries < (1u << 20)) return HB2_OK;
+        if (A->nslots + A->nlong_entries < (1u << 18)) return HB2_OK;
         T * x = nullptr, * y = nullptr;
         HB2_CUDA(cudaMalloc(&x, sizeof(T) * std::max<uint64_t>(A->cols, 1)));
         cudaError_t e = cudaMalloc(&y, sizeof(T) * std::max<uint64_t>(A->rows, 1));
@@ -323,10 +543,13 @@ namespace
         if (e == cudaSuccess) e = cudaEventCreate(&ev[1]);
         float best = 1e30f;
         int best_u = 8;
-        for (int u : {8, 16})
+        bool best_staged = false;
+        for (int v = 0; v < (A->win_bytes ? 4 : 2); ++v)
         {
+            const int u = v & 1 ? 16 : 8;
             if (e != cudaSuccess) break;
             A->unroll = u;
+            A->staged = v >= 2;
             int st = launch<T, false>(A, nullptr, x, y, stream);    // warm-up
             if (st) { e = cudaErrorUnknown; break; }
             e = cudaEventRecord(ev[0], stream);
@@ -336,9 +559,10 @@ namespace
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
             float ms = 0;
             if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev[0], ev[1]);
-            if (e == cudaSuccess && ms < best) { best = ms; best_u = u; }
+            if (e == cudaSuccess && ms < best) { best = ms; best_u = u; best_staged = A->staged; }
         }
         A->unroll = best_u;
+        A->staged = best_staged;
         if (ev[0]) cudaEventDestroy(ev[0]);
         if (ev[1]) cudaEventDestroy(ev[1]);
         cudaFree(x);
@@ -459,7 +683,32 @@ namespace
                     sval[slices[sl].x + H * k + j] = eval[start[r] + k];
                 }
             }
+        // each window's span of x; the staged kernel is a candidate when nine windows in ten fit
+        // and the long rows are few enough for a CTA each
+        const uint32_t nwindows = (uint32_t)((short_rows.size() + kSigma - 1) / kSigma);
+        std::vector<uint2> xwin(nwindows);
+        uint64_t span_max = 1;
+        uint32_t wide = 0;
+        for (uint32_t w = 0; w < nwindows; ++w)
+        {
+            int32_t lo = INT32_MAX, hi = -1;
+            for (size_t q = (size_t)w * kSigma; q < std::min<size_t>(short_rows.size(), (size_t)(w + 1) * kSigma); ++q)
+                for (uint64_t i = start[short_rows[q]]; i < start[short_rows[q] + 1]; ++i)
+                {
+                    lo = std::min(lo, ecol[i]);
+                    hi = std::max(hi, ecol[i]);
+                }
+            xwin[w] = hi < 0 ? make_uint2(0, 0) : make_uint2((uint32_t)lo, (uint32_t)(hi - lo + 1));
+            if ((uint64_t)xwin[w].y * sizeof(T) > kWinBytes)
+            {
+                xwin[w].y = kNoWindow;
+                ++wide;
+            }
+            else span_max = std::max<uint64_t>(span_max, xwin[w].y);
+        }
+        const bool fits = nwindows > 0 && wide <= nwindows / 10 && tasks.size() - 1 <= (size_t)num_sms();
         cudaError_t e = upload((void **)&A->slices, slices, stream);
+        if (e == cudaSuccess && fits) e = upload((void **)&A->xwin, xwin, stream);
         if (e == cudaSuccess) e = upload((void **)&A->perm, perm, stream);
         if (e == cudaSuccess) e = upload((void **)&A->scol, scol, stream);
         if (e == cudaSuccess) e = upload(&A->sval, sval, stream);
@@ -471,6 +720,8 @@ namespace
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_status(e, "hb2_csr_create upload");
         A->nslices = (uint32_t)nslices;
+        A->nwindows = nwindows;
+        A->win_bytes = fits ? (uint32_t)((span_max * sizeof(T) + 15) / 16 * 16) : 0;
         A->nslots = nslots;
         A->nitems = (uint32_t)items.size();
         A->nlong_warps = (uint32_t)tasks.size() - 1;
