@@ -318,6 +318,124 @@ namespace hb2
         }
     }
 
+    // The one-reduction recurrence of cg_warp_reg (kCgTreeOneReduction) on a 9 x 9 Q1 grid
+    // operator with equal couplings (interior diagonal v4, couplings v0, boundary diagonal vb),
+    // FP64 arithmetic, one warp.  A lane owns three rows of one column (27 lanes), so a product
+    // gathers 12 values instead of 27, keeps no matrix in registers and shares the line sums of
+    // its rows.  Bound by the dependent chain of an iteration (two warp sums, a reciprocal, the
+    // gather); measured (B200): 0.29 -> 0.26 us an iteration, a level-6 solve of 7 cycles 442 ->
+    // 419 us, of level 10 with 8 cycles 1,354 -> 1,289.  smem: 2 x 81 doubles.
+    template <typename S>
+    __device__ __forceinline__ void cg_warp_grid9(double v0, double v4, double vb, const S * b, S * xg, uint64_t max_iters,
+                                                  double eps, uint64_t * used_out, double * defect_out, double * smem)
+    {
+        typedef Arith<double> M;
+        constexpr int m = 9, R = 3;
+        const int lane = threadIdx.x & 31, j = lane % m, i0 = lane / m * R;
+        const bool live = lane < m * (m / R);
+        const int jw = max(j - 1, 0), je = min(j + 1, m - 1);
+        int at[R + 2];          // the lines around the lane's rows
+        bool edge[R];
+#pragma unroll
+        for (int k = 0; k < R + 2; ++k) at[k] = min(max(i0 + k - 1, 0), m - 1) * m;
+#pragma unroll
+        for (int k = 0; k < R; ++k) edge[k] = j == 0 || j == m - 1 || i0 + k == 0 || i0 + k >= m - 1;
+        auto product = [&](double (&out)[R], const double * v, const double (&own)[R]) {
+            double h[R + 2], H[R + 2];
+#pragma unroll
+            for (int k = 0; k < R + 2; ++k)
+            {
+                const double c = k >= 1 && k <= R ? own[k >= 1 && k <= R ? k - 1 : 0] : v[at[k] + j];
+                h[k] = M::add(v[at[k] + jw], v[at[k] + je]);
+                H[k] = M::add(h[k], c);
+            }
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+            {
+                const double s = M::fma(v0, M::add(M::add(H[k], H[k + 2]), h[k + 1]), M::mul(v4, own[k]));
+                out[k] = edge[k] ? M::mul(vb, own[k]) : s;
+            }
+        };
+        auto store = [&](double * v, const double (&a)[R]) {
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+                if (live) v[(i0 + k) * m + j] = a[k];
+        };
+        auto dot = [&](const double (&a)[R], const double (&c)[R]) -> double {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < R; ++k) s = fma(a[k], c[k], s);
+            return warp_sum_mma(live ? s : 0.0);
+        };
+        double * cur = smem, * nxt = smem + m * m;
+        double xr[R], rr[R], pr[R], sr[R], wr[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) xr[k] = live ? (double)xg[(i0 + k) * m + j] : 0.0;
+        store(cur, xr);
+        __syncwarp();
+        product(wr, cur, xr);
+#pragma unroll
+        for (int k = 0; k < R; ++k) pr[k] = rr[k] = live ? M::sub((double)b[(i0 + k) * m + j], wr[k]) : 0.0;
+        store(nxt, rr);
+        __syncwarp();
+        double g = dot(rr, rr);
+        const double initial = sqrt(g);
+        double current = initial;
+        uint64_t it = 0, used = 0;
+        if (max_iters > 0)
+        {
+            product(wr, nxt, rr);
+            double a = M::div(g, guard(dot(wr, rr)));
+            double inv_a = Recip<double>::rn(guard(a)), inv_g = Recip<double>::rn(guard(g));
+            const double thr = M::mul(eps, initial), thr2 = M::mul(thr, thr), eps2 = M::mul(eps, eps);
+            const double inv_eps = Recip<double>::rn(Eps<double>::v());
+#pragma unroll
+            for (int k = 0; k < R; ++k) sr[k] = wr[k];
+            while (true)
+            {
+#pragma unroll
+                for (int k = 0; k < R; ++k) rr[k] = M::fma(-a, sr[k], rr[k]);
+                store(cur, rr);
+                __syncwarp();
+                g = dot(rr, rr);
+                product(wr, cur, rr);
+#pragma unroll
+                for (int k = 0; k < R; ++k) xr[k] = M::fma(a, pr[k], xr[k]);
+                double * t = cur;
+                cur = nxt;
+                nxt = t;
+                const double del = dot(wr, rr);
+                ++it;
+                const double bt = M::mul(g, inv_g), bg = M::mul(M::mul(bt, g), inv_a);
+                const double ig = Recip<double>::rn(guard(g));
+#pragma unroll
+                for (int k = 0; k < R; ++k)
+                {
+                    pr[k] = M::fma(bt, pr[k], rr[k]);
+                    sr[k] = M::fma(bt, sr[k], wr[k]);
+                }
+                if (g < thr2 || g < eps2 || it == max_iters)
+                {
+                    current = sqrt(g);
+                    used = it;
+                    break;
+                }
+                const double d = guard(M::sub(del, bg));
+                a = M::mul(g, Recip<double>::rn(d));
+                inv_g = ig;
+                inv_a = fabs(a) > Eps<double>::v() ? M::mul(d, ig) : inv_eps;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (live) xg[(i0 + k) * m + j] = S(xr[k]);
+        if (lane == 0)
+        {
+            if (used_out) *used_out = used;
+            if (defect_out) *defect_out = current;
+        }
+    }
+
     template <typename T, typename S, int RPL>
     __global__ void __launch_bounds__(32)
     cg_warp_reg_kernel(EllView<T> Ag, const S * __restrict__ b, S * __restrict__ xg, uint64_t max_iters, double eps_d,

@@ -35,6 +35,8 @@ namespace hb2
         EllView<T> C;                               // coarsest operator
         EllView<double> C64;                        // its FP64 copy (mixed)
         int mixed, exact;
+        int grid9;                                  // the coarsest is a 9 x 9 Q1 grid operator with equal
+        double cv0, cv4, cvb;                       // couplings, solved in FP64 by cg_warp_grid9
         uint64_t max_iters;
         double eps;
         uint64_t * used;
@@ -217,7 +219,9 @@ namespace hb2
             ts[l] = r;          // xs: the iterate, ts: free
             xs[l] = cur;
         }
-        if (threadIdx.x < 32)
+        if (threadIdx.x < 32 && g.grid9)
+            cg_warp_grid9<T>(g.cv0, g.cv4, g.cvb, bs[0], xs[0], g.max_iters, g.eps, g.used, g.defect, cgs);
+        else if (threadIdx.x < 32)
         {
             if constexpr (MIXED)
                 bottom_coarse<double, T>(g.C64, bs[0], xs[0], g.max_iters, g.eps, g.exact, g.used, g.defect, cgs);
@@ -269,6 +273,14 @@ namespace hb2
         g.C = p.A[0]->view<T>();
         if (p.coarse64) g.C64 = p.coarse64->view<double>();
         g.exact = p.exact;
+        // FP64 and the reordered recurrence only: the other modes sum in a given order.  Of the
+        // sizes that fit one warp 9 x 9 is the one a hierarchy ends on by default (level 3).
+        const hb2_ell_s * C = p.coarse64 ? p.coarse64 : p.A[0];
+        g.grid9 = C->dtype == HB2_F64 && C->q1g_m == 9 && p.exact == kCgTreeOneReduction;
+        for (int k = 0; k < 9; ++k) g.grid9 = g.grid9 && (k == 4 || C->q1g_v[k] == C->q1g_v[0]);
+        g.cv0 = C->q1g_v[0];
+        g.cv4 = C->q1g_v[4];
+        g.cvb = C->q1g_vb;
         g.max_iters = p.max_iters;
         g.eps = p.eps;
         g.used = p.used;

@@ -83,3 +83,29 @@ def test_cycle_matches_single_passes(monkeypatch, coarse, level, dt, pre, post, 
     assert np.array_equal(out[0][0].view(np.uint8), out[1][0].view(np.uint8))
     # the norms: sums of m^2 squares in two orders, each at most m^2 eps off relative to the sum
     assert abs(out[0][1] / out[1][1] - 1.0) <= m * m * 2.0 ** -52
+
+
+# The coarse CG on a 9 x 9 Q1 grid operator with equal couplings, three rows of one column a lane
+# (cg_warp_grid9), against the one that gathers from the ELL matrix; aniso != 1 and a coarsest of
+# another size keep the latter on both sides.  caps: no step, one, fewer and more than it takes.
+@pytest.mark.parametrize("coarse,aniso", [(3, 1.0), (3, 2.0), (2, 1.0)])
+@pytest.mark.parametrize("cap", [0, 1, 7, 100])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_coarse_cg_on_the_grid(monkeypatch, coarse, aniso, cap, mixed):
+    dt = torch.float32 if mixed else torch.float64
+    m = 33
+    i = torch.arange(m * m, device="cuda", dtype=torch.float64)
+    out = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("HB2_Q1_TRANSFER", flag)
+        data = hb.MGData.poisson_q1(coarse, 5, dtype=dt, aniso=aniso,
+                                    params=hb.mg_params(4, 4, max_iters=2, max_iters_coarse=cap, eps=1e-30,
+                                                        coarse_exact=False, coarse_fp64=mixed))
+        x = DenseVector(torch.zeros(m * m, device="cuda", dtype=dt))
+        hb.MGSolver.value(data, DenseVector(torch.sin(i).to(dt)), x)
+        out.append(x.numpy().astype(np.float64))
+    # a coarse solution differs by at most steps x condition (below 64 on 9 x 9) x 2^-52; two cycles
+    # add one such correction each.  Stored in FP32 it may round to the neighbour, and then so may
+    # each of the at most 24 sweeps and transfers of a cycle behind it.
+    u = 2.0 ** -52 * 100 * 64 + (24 * 2.0 ** -23 if mixed else 0.0)
+    assert np.abs(out[0] - out[1]).max() <= 2 * 2 * u * np.abs(out[1]).max()
