@@ -240,7 +240,8 @@ namespace
         cp_async_wait_pending<0>();
     }
 
-    // The long rows of one warp alone in its CTA.  The chain over a chunk (128 dependent fma, 0.3
+    // A task's long rows in a CTA of their own: warp 0 runs the chain, warp 1 keeps it fed (one
+    // warp doing both took 1,400 cycles a chunk, twice the chain).  The chain over a chunk (128 dependent fma, 0.3
     // us in FP32) is far shorter than what stands behind a chunk -- its item, its columns, the x
     // they name, each a load that needs the one before -- so all three run ahead of it: items by
     // the warp's lanes (32 at a time), columns by cp.async kDeepL chunks before they are used,
@@ -250,7 +251,7 @@ namespace
     template <typename T> constexpr size_t deep_bytes() { return kDeepS * 2 * kW * sizeof(T) + kDeepC * kW * sizeof(int32_t); }
 
     template <typename T, bool DEFECT>
-    __device__ __forceinline__ void run_long_deep(uint32_t k0, uint32_t k1, uint32_t lane, unsigned char * smem,
+    __device__ __forceinline__ void run_long_deep(uint32_t k0, uint32_t k1, uint32_t warp, uint32_t lane, unsigned char * smem,
                                                   const uint4 * __restrict__ items, const int32_t * __restrict__ lcol,
                                                   const T * __restrict__ lval, const T * __restrict__ x,
                                                   const T * __restrict__ rhs, T * __restrict__ y)
@@ -291,13 +292,16 @@ namespace
                 }
             }
         };
-        for (uint32_t q = 0; q < kDeepS - 1 + kDeepL; ++q) columns(k0 + q);
-        cp_async_commit();
-        cp_async_wait_pending<0>();
-        for (uint32_t q = 0; q < kDeepS - 1; ++q)
+        if (warp == 1)
         {
-            stage(k0 + q);
+            for (uint32_t q = 0; q < kDeepS - 1 + kDeepL; ++q) columns(k0 + q);
             cp_async_commit();
+            cp_async_wait_pending<0>();
+            for (uint32_t q = 0; q < kDeepS - 1; ++q)
+            {
+                stage(k0 + q);
+                cp_async_commit();
+            }
         }
         T s = T(0);
         for (uint32_t k = k0; k < k1; ++k)
@@ -308,11 +312,16 @@ namespace
                 i0 = i1;
                 i1 = kb + 32 + lane < k1 ? __ldg(items + kb + 32 + lane) : none;
             }
-            cp_async_wait_pending<kDeepS - 2>();
-            __syncwarp();                      // chunk k is here, chunk k - 1 is done with
-            stage(k + kDeepS - 1);
-            columns(k + kDeepS - 1 + kDeepL);
-            cp_async_commit();
+            if (warp == 1) cp_async_wait_pending<kDeepS - 2>();
+            // both warps, once a chunk: chunk k is here, chunk k - 1 is done with
+            asm volatile("bar.sync 1, 64;" ::: "memory");
+            if (warp == 1)
+            {
+                stage(k + kDeepS - 1);
+                columns(k + kDeepS - 1 + kDeepL);
+                cp_async_commit();
+                continue;
+            }
             const uint4 it = item(k);
             if (lane == 0)
             {
@@ -363,33 +372,41 @@ namespace
         cp_async_wait_pending<0>();
     }
 
-    template <typename T, bool DEFECT, int U>
+    // How the long rows run: a kernel without them keeps their registers and shared memory out of
+    // the slices' occupancy (level-11 Q1 operator, FP64: 105 us; with the deep form compiled in 115)
+    enum LongRows { kNoLong = 0, kLongShared = 1, kLongDeep = 2 };
+
+    template <typename T, bool DEFECT, int U, int LONG>
     __global__ void __launch_bounds__(32 * kCsrWarps) csr_kernel(
-        uint32_t long_ctas, int deep, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
+        uint32_t long_ctas, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
         uint32_t nlong_warps, const int32_t * __restrict__ lcol, const T * __restrict__ lval,
         const uint2 * __restrict__ slices, uint32_t nslices, const uint32_t * __restrict__ perm,
         const int32_t * __restrict__ scol, const T * __restrict__ sval, const T * __restrict__ x,
         const T * __restrict__ rhs, T * __restrict__ y)
     {
-        // the long rows' buffers: [warp][buffer][value | x][i], or those of one warp (run_long_deep)
-        constexpr size_t kBytes = kCsrWarps * 2 * 2 * kW * sizeof(T);
-        __shared__ __align__(16) unsigned char sbuf[deep_bytes<T>() > kBytes ? deep_bytes<T>() : kBytes];
         const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (blockIdx.x < long_ctas)
+        if constexpr (LONG != kNoLong)
         {
-            if (deep)
+            if (blockIdx.x < long_ctas)
             {
-                if (warp == 0)
-                    run_long_deep<T, DEFECT>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), lane, sbuf, items, lcol,
-                                             lval, x, rhs, y);
+                if constexpr (LONG == kLongDeep)
+                {
+                    // one task per CTA, on two of its warps
+                    __shared__ __align__(16) unsigned char dbuf[deep_bytes<T>()];
+                    if (warp < 2)
+                        run_long_deep<T, DEFECT>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), warp, lane, dbuf,
+                                                 items, lcol, lval, x, rhs, y);
+                }
+                else
+                {
+                    __shared__ __align__(16) T sbuf[kCsrWarps][2][2][kW];     // [warp][buffer][value | x][i]
+                    const uint32_t w = blockIdx.x * kCsrWarps + warp;
+                    if (w < nlong_warps)
+                        run_long<T, DEFECT, 2>(__ldg(tasks + w), __ldg(tasks + w + 1), lane, sbuf[warp], items, lcol, lval, x,
+                                               rhs, y);
+                }
                 return;
             }
-            const uint32_t w = blockIdx.x * kCsrWarps + warp;
-            if (w < nlong_warps)
-                run_long<T, DEFECT, 2>(__ldg(tasks + w), __ldg(tasks + w + 1), lane,
-                                       reinterpret_cast<T (*)[2][kW]>(sbuf) + 2 * warp, items, lcol, lval, x,
-                                    rhs, y);
-            return;
         }
         const uint32_t slice = (blockIdx.x - long_ctas) * kCsrWarps + warp;
         if (slice < nslices) run_slice<T, DEFECT, U>(slice, lane, slices, perm, scol, sval, x, rhs, y);
@@ -399,8 +416,8 @@ namespace
     // memory.  Gathers whose lanes fall on many cache lines cost the L1 one line each -- about
     // 28 cycles a warp on random columns near the diagonal, 21 of the 25 us of a product with
     // 7 million of them -- where shared memory pays bank conflicts only.  The long rows' CTAs
-    // come first, as in csr_kernel, one warp each.
-    template <typename T, bool DEFECT, int U>
+    // come first, as in csr_kernel.
+    template <typename T, bool DEFECT, int U, int LONG>
     __global__ void __launch_bounds__(32 * kWinWarps, 2) csr_staged_kernel(
         uint32_t long_ctas, const uint4 * __restrict__ items, const uint32_t * __restrict__ tasks,
         const int32_t * __restrict__ lcol, const T * __restrict__ lval, const uint2 * __restrict__ xwin,
@@ -410,13 +427,16 @@ namespace
     {
         extern __shared__ __align__(16) unsigned char csr_smem[];
         const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (blockIdx.x < long_ctas)
+        if constexpr (LONG != kNoLong)
         {
-            __shared__ __align__(16) unsigned char lbuf[deep_bytes<T>()];
-            if (warp == 0)
-                run_long_deep<T, DEFECT>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), lane, lbuf, items, lcol, lval,
-                                         x, rhs, y);
-            return;
+            if (blockIdx.x < long_ctas)
+            {
+                __shared__ __align__(16) unsigned char lbuf[deep_bytes<T>()];
+                if (warp < 2)
+                    run_long_deep<T, DEFECT>(__ldg(tasks + blockIdx.x), __ldg(tasks + blockIdx.x + 1), warp, lane, lbuf, items,
+                                             lcol, lval, x, rhs, y);
+                return;
+            }
         }
         T * xs = reinterpret_cast<T *>(csr_smem);
         const uint32_t w = blockIdx.x - long_ctas, slice = w * kWinWarps + warp;
@@ -489,15 +509,17 @@ namespace
     template <typename T, bool DEFECT>
     int launch(hb2_csr A, const void * rhs, const void * x, void * y, cudaStream_t stream)
     {
-        // few long rows: each warp alone in its CTA, eight chunks deep;
+        // few long rows: each task in a CTA of its own, eight chunks deep;
         // with more of them than SMs the four-warp form keeps more chains resident
         const int deep = A->nlong_warps <= (uint32_t)num_sms();
         const uint32_t long_ctas = deep ? A->nlong_warps : (A->nlong_warps + kCsrWarps - 1) / kCsrWarps;
         const uint32_t slice_ctas = (A->nslices + kCsrWarps - 1) / kCsrWarps;
         if (long_ctas + slice_ctas == 0) return HB2_OK;
+        const int mode = A->nlong_warps == 0 ? kNoLong : deep ? kLongDeep : kLongShared;
         if (A->staged)
         {
-            auto ks = A->unroll == 16 ? csr_staged_kernel<T, DEFECT, 16> : csr_staged_kernel<T, DEFECT, 8>;
+            auto ks = mode == kNoLong ? (A->unroll == 16 ? csr_staged_kernel<T, DEFECT, 16, kNoLong> : csr_staged_kernel<T, DEFECT, 8, kNoLong>)
+                                      : (A->unroll == 16 ? csr_staged_kernel<T, DEFECT, 16, kLongDeep> : csr_staged_kernel<T, DEFECT, 8, kLongDeep>);
             HB2_CUDA(cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->win_bytes));
             ks<<<A->nlong_warps + A->nwindows, 32 * kWinWarps, A->win_bytes, stream>>>(
                 A->nlong_warps, A->items, A->tasks, A->lcol, (const T *)A->lval, A->xwin, A->slices, A->nslices, A->perm,
@@ -506,9 +528,12 @@ namespace
             HB2_LAUNCH_CHECK("csr_staged_kernel");
             return HB2_OK;
         }
-        auto k = A->unroll == 16 ? csr_kernel<T, DEFECT, 16> : csr_kernel<T, DEFECT, 8>;
+        const bool u16 = A->unroll == 16;
+        auto k = mode == kNoLong     ? (u16 ? csr_kernel<T, DEFECT, 16, kNoLong> : csr_kernel<T, DEFECT, 8, kNoLong>)
+                 : mode == kLongDeep ? (u16 ? csr_kernel<T, DEFECT, 16, kLongDeep> : csr_kernel<T, DEFECT, 8, kLongDeep>)
+                                     : (u16 ? csr_kernel<T, DEFECT, 16, kLongShared> : csr_kernel<T, DEFECT, 8, kLongShared>);
         k<<<long_ctas + slice_ctas, 32 * kCsrWarps, 0, stream>>>(
-            long_ctas, deep, A->items, A->tasks, A->nlong_warps, A->lcol, (const T *)A->lval, A->slices, A->nslices,
+            long_ctas, A->items, A->tasks, A->nlong_warps, A->lcol, (const T *)A->lval, A->slices, A->nslices,
             A->perm, A->scol, (const T *)A->sval, (const T *)x, (const T *)rhs, (T *)y);
         count_launches(1);
         HB2_LAUNCH_CHECK("csr_kernel");
@@ -631,7 +656,7 @@ namespace
         std::vector<uint32_t> tasks;
         {
             int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csr_kernel<T, false, 8>, 32 * kCsrWarps, 0) !=
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csr_kernel<T, false, 8, kLongShared>, 32 * kCsrWarps, 0) !=
                     cudaSuccess || per_sm < 1)
                 per_sm = 1;
             const uint64_t nwarps = std::max<uint64_t>(1, std::min<uint64_t>(nlong_rows, (uint64_t)per_sm * num_sms() * kCsrWarps));
