@@ -41,7 +41,6 @@ COARSE_CAP = 100
 MIXED_LEVEL = 11
 DEFAULT_LEVEL = 11
 SERVING_RATES = (50.0, 100.0, 200.0, 500.0, 1000.0, 2000.0)
-SUB_MAX_ROWS = 20000    # levels up to this many rows run in the fused small-level kernels
 
 
 def parse():
@@ -87,22 +86,22 @@ def mg_solve_bytes(level: int, cycles: int, row_bytes, min_level: int = MIN_LEVE
     return cycles * total + nF * (row_bytes(level, "A") + 3 * s)
 
 
-def layout_row_bytes(hb, dtype, levels):
-    """row_bytes(l, which) for mg_solve_bytes, from matrices of the same shapes as the
-    hierarchy's (the layout choice is made once per shape and process)."""
-    import torch
-    # levels above SUB_MAX_ROWS rows apply their transfers with the Q1 transfer kernels,
-    # which read no matrix (unless HB2_Q1_TRANSFER=0); the fused small levels read them
-    q1t = os.environ.get("HB2_Q1_TRANSFER", "1") != "0"
-    table = {}
-    for l in levels:
-        table[(l, "A")] = hb.SparseMatrixELL.poisson_q1(l, dtype).layout()[2]
-        if l > min(levels):
-            P, R = hb.SparseMatrixELL.transfer(l, dtype)
-            table[(l, "P")], table[(l, "R")] = P.layout()[2], R.layout()[2]
-            if q1t and ((1 << l) + 1) ** 2 > SUB_MAX_ROWS:
-                table[(l, "P")] = table[(l, "R")] = 0
-    return lambda l, which: table[(l, which)]
+def mg_sweep_bytes(level: int, cycles: int, min_level: int = MIN_LEVEL, s: int = 8) -> int:
+    """Algorithmic HBM bytes of one MG solve in Q1 sweep passes (V(n, n), n <= 4), each vector
+    touched once per pass: down, the finest level reads x and b, a coarser one b only, and
+    writes x and the coarser right-hand side; up, x, b and the coarser correction in, x out.
+    Levels of at most 33 points a line run in one block (b in, x out).  Plus the initial
+    defect."""
+    total = 0
+    for l in range(min_level + 1, level + 1):
+        nf = ((1 << l) + 1) ** 2
+        nc = ((1 << (l - 1)) + 1) ** 2
+        if (1 << l) + 1 <= 33:
+            total = 2 * nf * s                       # the bottom: its largest level's vectors only
+            continue
+        total += nf * s * (3 if l == level else 2) + nc * s
+        total += nf * s * 3 + nc * s
+    return cycles * total + 3 * s * ((1 << level) + 1) ** 2
 
 
 JACOBI_BYTES_PER_ROW = 9 * (8 + 4) + 4 * 8     # FP64 values, int32 columns: 140 B
@@ -264,7 +263,7 @@ def workload_config(args, world):
 ROW_BYTES = {"jacobi": 4, "spmv": 2, "defect": 3}   # vector accesses per row (8 B each in FP64)
 
 
-def kernel_roofline(hb, kind, A, level, peak, dev, reps=12, label=None, dtype=None, key_suffix=""):
+def kernel_roofline(hb, kind, A, level, peak, dev, reps=12, label=None, dtype=None, key_suffix="", row_bytes=None):
     """One ELL kernel of the level-`level` operator on the layout A runs on, timed in
     its steady state: 40 launches captured in one CUDA graph, rotating over sets of
     input and output vectors of more than 2x L2 in all (every launch reads its vectors
@@ -282,6 +281,10 @@ def kernel_roofline(hb, kind, A, level, peak, dev, reps=12, label=None, dtype=No
     kind_l, table_size, rb = A.layout()
     vk, vr, vw = A.layout_variant(1 if kind == "defect" else 0)
     variant = variant_name(vk, vr, vw)
+    if kind != "jacobi" and variant.startswith("q1") and level >= 8:
+        # products and defects of a Q1 grid operator stream x (and b) only, no matrix bytes
+        variant, rb = "q1stream", 0
+    rb = rb if row_bytes is None else row_bytes
     nbytes = n * (rb + es * ROW_BYTES[kind])
     achieved = nbytes / (ms * 1e-3) / 1e9
     key = f"{variant}:{kind}:L{level}{key_suffix}"
@@ -402,8 +405,7 @@ def main():
     peaks = load_peaks()
     roof = kernel_roofline(hb, "jacobi", A, L, peaks, dev,
                            label=f"fused Jacobi sweep x' = x + P (b - A x), level {L}, FP64")
-    solve_bytes = mg_solve_bytes(L, int(statistics.median(cycles)),
-                                 layout_row_bytes(hb, torch.float64, range(MIN_LEVEL, L + 1)))
+    solve_bytes = mg_sweep_bytes(L, int(statistics.median(cycles)))
     line = {
         "metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": mean_ms_max, "higher_is_better": True, "scaling": "weak",
@@ -754,6 +756,8 @@ def bf16_variant(hb, dev, flush, level, peaks, rank):
         for name, M in finest.items():
             kr = kernel_roofline(hb, "jacobi", M, level, peaks, dev, dtype=torch.float32,
                                  label=f"fused Jacobi sweep, level {level}, {op} operator, {name} inner matrix",
+                                 # the coefficient operator's FP32 rows are read without their columns
+                                 row_bytes=36 if op != "q1" and name == "fp32" else None,
                                  key_suffix="" if op == "q1" else
                                  ":coefficients" + ("" if name == "fp32" else "-" + name.split("_")[1]))
             rep[name]["sweep"] = {key: kr[key] for key in ("variant", "launch_shape", "bytes_per_row", "launch_us",

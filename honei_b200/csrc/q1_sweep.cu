@@ -136,7 +136,7 @@ namespace hb2
     // Product, defect (+ norm) and product with dot of a large Q1 grid operator as streaming
     // passes.  From 2^16 rows up: below, the one-row-per-thread kernels are as fast and their
     // layout was timed at creation.  Measured (B200), FP64 level 11: defect + norm 37.2 us
-    // with the gather kernel.
+    // with the gather kernel, 26.6 as a streaming pass (a call, partial sums included).
     bool q1_single_applies(const hb2_ell_s * A, int mode)
     {
         return A->q1g_m >= 257 && (mode == kPlain || mode == kDefect || mode == kDot);
