@@ -373,7 +373,7 @@ namespace
     }
 
     // How the long rows run: a kernel without them keeps their registers and shared memory out of
-    // the slices' occupancy (level-11 Q1 operator, FP64: 105 us; with the deep form compiled in 115)
+    // the slices' occupancy (level-11 Q1 operator, FP64: 106 us, with the deep form compiled in 115)
     enum LongRows { kNoLong = 0, kLongShared = 1, kLongDeep = 2 };
 
     template <typename T, bool DEFECT, int U, int LONG>
