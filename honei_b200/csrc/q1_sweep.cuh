@@ -34,6 +34,7 @@
 
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
+#include "smem_opt_in.hh"
 
 #include <algorithm>
 #include <type_traits>
@@ -521,7 +522,7 @@ namespace hb2
         g.bpv = (g.strips * g.chunks + kSweepWarps - 1) / kSweepWarps;
         const size_t smem = K::ring(PVEC) * sizeof(T) * kSweepWarps;
         auto kern = q1_sweep_kernel<T, C, UNI, S, HEAD, TAIL, PVEC>;
-        static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t attr = smem_opt_in((const void *)kern, smem);
         if (attr != cudaSuccess) return cuda_status(attr, "Q1 sweep kernel: shared memory");
         uint64_t grid = (uint64_t)g.bpv * (g.list ? max_vec : 1);
         if (g.list && cap) grid = std::min(grid, cap);
