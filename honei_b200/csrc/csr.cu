@@ -29,6 +29,7 @@
 // then the slices.  The reference arrays are kept on the host for export.
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
+#include "smem_opt_in.hh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -520,7 +521,8 @@ namespace
         {
             auto ks = mode == kNoLong ? (A->unroll == 16 ? csr_staged_kernel<T, DEFECT, 16, kNoLong> : csr_staged_kernel<T, DEFECT, 8, kNoLong>)
                                       : (A->unroll == 16 ? csr_staged_kernel<T, DEFECT, 16, kLongDeep> : csr_staged_kernel<T, DEFECT, 8, kLongDeep>);
-            HB2_CUDA(cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->win_bytes));
+            // the largest window's size, not this matrix's: the limit is the kernel's, shared by all matrices
+            HB2_CUDA(smem_opt_in((const void *)ks, kWinBytes));
             ks<<<A->nlong_warps + A->nwindows, 32 * kWinWarps, A->win_bytes, stream>>>(
                 A->nlong_warps, A->items, A->tasks, A->lcol, (const T *)A->lval, A->xwin, A->slices, A->nslices, A->perm,
                 A->scol, (const T *)A->sval, (const T *)x, (const T *)rhs, (T *)y);

@@ -1,0 +1,78 @@
+"""Two host threads, each on its own stream, and two live handles that share a kernel: what
+one of them needs (a kernel's shared-memory limit) must not be taken away by the other.  Every call is held to the bits that it gives alone."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+import honei_b200 as hb
+from honei_b200 import _lib
+from honei_b200 import DenseVector, SparseMatrixCSR
+from honei_b200.inputs import uniform
+
+pytestmark = pytest.mark.gpu
+
+
+def dvec(a):
+    return DenseVector(torch.from_numpy(np.ascontiguousarray(a)).cuda())
+
+
+def in_threads(*work):
+    """Runs the callables at the same time, each on a stream of its own; their results."""
+    out, errors = [None] * len(work), []
+    start = threading.Barrier(len(work))
+
+    def body(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                out[i] = work[i]()
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:          # re-raised below, in the test's thread
+            errors.append(e)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=body, args=(i,)) for i in range(len(work))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    if errors:
+        raise errors[0]
+    return out
+
+
+@pytest.mark.parametrize("npdt", [np.float64, np.float32])
+def test_csr_products_of_different_windows(monkeypatch, npdt):
+    """Staged products whose windows of x are some 5 KiB and just below 64 KiB."""
+    monkeypatch.setenv("HB2_CSR_U", "8")
+    monkeypatch.setenv("HB2_CSR_STAGED", "1")
+    rows = 4096
+    rng = np.random.default_rng(1)
+
+    def make(spread):
+        ar = np.arange(rows + 1, dtype=np.int64) * 8
+        row = np.repeat(np.arange(rows), 8)
+        aj = np.clip(row + rng.integers(-spread, spread + 1, row.size), 0, rows + 16000)
+        return SparseMatrixCSR.from_arrays(rows, rows + 16001, ar, aj, uniform(row.size, 3, dtype=npdt))
+    # a window spans 512 + 2 spread columns
+    mats = [make(40), make((65536 // np.dtype(npdt).itemsize - 600) // 2)]
+    x = dvec(uniform(rows + 16001, 4, dtype=npdt))
+    ys = [dvec(np.zeros(rows, npdt)) for _ in mats]
+
+    # straight through the C ABI: the two threads' calls have to meet inside the library
+    product = _lib.load().hb2_product_csr
+
+    def products(k, count=20000):
+        s = torch.cuda.current_stream().cuda_stream
+        args = (mats[k].handle, ctypes.c_void_p(x.ptr.value), ctypes.c_void_p(ys[k].ptr.value), ctypes.c_void_p(s))
+        for i in range(count):
+            assert product(*args) == 0, (i, _lib.load().hb2_last_error())
+    alone = []
+    for k in (0, 1):
+        products(k, 1)
+        alone.append(ys[k].numpy().copy())
+    in_threads(lambda: products(0), lambda: products(1))
+    for k in (0, 1):
+        assert np.array_equal(ys[k].numpy().view(np.uint8), alone[k].view(np.uint8))
