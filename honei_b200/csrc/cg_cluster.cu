@@ -13,6 +13,7 @@
 // sums, one value per CTA written to every CTA's shared memory, and summed by each warp in rank
 // order, so all CTAs hold the same bits and leave the loop together.
 #include "cg_warp.cuh"
+#include "smem_opt_in.hh"
 
 #include <cooperative_groups.h>
 
@@ -187,7 +188,7 @@ namespace hb2
     {
         const size_t smem = ((size_t)(g.lines + 4) * g.m) * sizeof(T) + 16;
         auto kern = cg_cluster_kernel<T, E>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = smem_opt_in((const void *)kern, smem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};

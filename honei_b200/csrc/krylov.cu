@@ -21,6 +21,7 @@
 // iteration counts may differ by one).  FP64.
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
+#include "smem_opt_in.hh"
 
 #include "cg_warp.cuh"
 
@@ -716,7 +717,7 @@ namespace
     cudaError_t launch_loop_e(const LoopArgs & g, cudaStream_t s)
     {
         const size_t smem = 4 * sizeof(double) * (size_t)g.rows * kLoopThreads;
-        cudaError_t e = cudaFuncSetAttribute(k_cg_loop<KT, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = smem_opt_in((const void *)k_cg_loop<KT, E>, smem);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)ceil_div(g.n, (uint64_t)g.rows * kLoopThreads));

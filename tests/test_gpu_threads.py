@@ -9,8 +9,8 @@ import torch
 
 import honei_b200 as hb
 from honei_b200 import _lib
-from honei_b200 import DenseVector, SparseMatrixCSR
-from honei_b200.inputs import uniform
+from honei_b200 import DenseVector, SparseMatrixCSR, SparseMatrixELL
+from honei_b200.inputs import q1_coefficient_operator, uniform
 
 pytestmark = pytest.mark.gpu
 
@@ -76,3 +76,43 @@ def test_csr_products_of_different_windows(monkeypatch, npdt):
     in_threads(lambda: products(0), lambda: products(1))
     for k in (0, 1):
         assert np.array_equal(ys[k].numpy().view(np.uint8), alone[k].view(np.uint8))
+
+
+def test_cluster_cg_of_different_sizes():
+    """Solves on clusters with slabs of different size; a launch refused for want of shared
+    memory would fall to another form, with other sums."""
+    A = [SparseMatrixELL.poisson_q1(level) for level in (6, 7, 8)]
+    b = [dvec(uniform(a.rows(), 3)) for a in A]
+    x = [dvec(np.zeros(a.rows())) for a in A]
+
+    def solves(k, count=20):
+        out = None
+        for _ in range(count):
+            hb.fill(x[k], 0.0)
+            out = hb.CGSolver.value(A[k], None, b[k], x[k], 60, eps_relative=1e-8)
+        return out[1:]
+    alone, bits = [], []
+    for k in range(3):
+        alone.append(solves(k, 1))
+        bits.append(x[k].numpy().copy())
+    together = in_threads(*[lambda k=k: solves(k) for k in range(3)])
+    for k in range(3):
+        assert together[k] == alone[k]
+        assert np.array_equal(x[k].numpy().view(np.uint8), bits[k].view(np.uint8))
+
+
+# 5 and 7 rows a thread: one instance of the loop kernel with 80 and 112 KiB of shared memory
+@pytest.mark.parametrize("order", [(700, 600), (600, 700)])
+def test_two_krylov_solvers_of_one_instance(order):
+    def make(cells):
+        op = q1_coefficient_operator(np.power(4.0, uniform(cells * cells, 5, -0.5, 0.5)).reshape(cells, cells))
+        A = SparseMatrixELL.from_arrays(*op)
+        P = hb.RISmoother.jacobi_precon(A, 1.0)
+        return hb.KrylovSolver(hb.HB2_CG_VAR, A, P, 10, 0.0), dvec(uniform(op[0], 42)), op[0]
+    first = make(order[0])
+    alone = first[0].solve(first[1], dvec(np.zeros(first[2])))[0].numpy().copy()
+    second = make(order[1])
+    for s in (first, second, first):
+        x = s[0].solve(s[1], dvec(np.zeros(s[2])))[0].numpy()
+        if s is first:
+            assert np.array_equal(x.view(np.uint8), alone.view(np.uint8))

@@ -25,7 +25,7 @@ def test_helper(tmp_path):
     assert res.returncode == 0 and res.stdout.strip() == "ok", res.stdout
 
 
-@pytest.mark.parametrize("source", ["q1_sweep.cuh", "csr.cu"])
+@pytest.mark.parametrize("source", ["q1_sweep.cuh", "csr.cu", "cg_cluster.cu", "krylov.cu"])
 def test_launches_go_through_the_helper(source):
     text = open(os.path.join(CSRC, source)).read()
     assert "smem_opt_in(" in text
