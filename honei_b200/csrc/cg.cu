@@ -16,6 +16,7 @@
 #include "cg_warp.cuh"
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
+#include "smem_opt_in.hh"
 
 #include <algorithm>
 #include <cfloat>
@@ -320,15 +321,10 @@ namespace hb2
         const bool mat = small_smem(A, true) <= kSmallSmemLimit;
         const size_t smem = small_smem(A, mat);
         int threads = (int)std::min<uint64_t>(1024, (A->rows + 31) / 32 * 32);
-        static bool attr_set = false;   // once per process, never inside a stream capture
-        if (! attr_set)
-        {
-            HB2_CUDA(cudaFuncSetAttribute(cg_small_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmemLimit + 64));
-            HB2_CUDA(cudaFuncSetAttribute(cg_small_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmemLimit + 64));
-            HB2_CUDA(cudaFuncSetAttribute(cg_warp_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmemLimit + 64));
-            HB2_CUDA(cudaFuncSetAttribute(cg_warp_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmemLimit + 64));
-            attr_set = true;
-        }
+        // once per device, at the largest size (creation calls this outside a stream capture)
+        for (const void * k : {(const void *)cg_small_kernel<double>, (const void *)cg_small_kernel<float>,
+                               (const void *)cg_warp_kernel<double>, (const void *)cg_warp_kernel<float>})
+            HB2_CUDA(smem_opt_in(k, kSmallSmemLimit + 64));
         // the register kernel for the 9-slot operators; others take the shared-memory one
         const bool reg = A->K != 9 ? false
                        : A->dtype == HB2_F64

@@ -25,6 +25,7 @@
 // computes from global memory instead (same bits) and records the event.
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
+#include "smem_opt_in.hh"
 #include "tma.cuh"
 
 #include <cstdlib>
@@ -552,19 +553,7 @@ namespace hb2
                                   int flags)
     {
         constexpr size_t smem = q1_stencil_smem<T, R>();
-        if (smem > 48 * 1024)
-        {
-            // dynamic shared memory above 48 KiB needs the kernel's opt-in, once per device
-            static bool done[64] = {};
-            int dev = 0;
-            cudaGetDevice(&dev);
-            if (dev >= 0 && dev < 64 && ! done[dev])
-            {
-                cudaFuncSetAttribute(q1_stencil_kernel<T, MODE, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
-                done[dev] = true;
-            }
-        }
+        if (smem > 48 * 1024) smem_opt_in((const void *)q1_stencil_kernel<T, MODE, R>, smem);    // the launch reports a refusal
         launch_pdl(q1_stencil_kernel<T, MODE, R>, grid, dim3(kEllThreads), smem, st, s, (const T *)x, (T *)y,
                    (const T *)aux, (const T *)aux2, rs, red, want_sqrt, flags);
     }

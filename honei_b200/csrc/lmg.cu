@@ -484,9 +484,7 @@ namespace
         g.konv_rad = (double)std::numeric_limits<T>::epsilon();
         g.mk = make_mask(G->prm.macro_border_mask);
         g.st = G->st;
-        const size_t smem = elems * sizeof(T);
-        if (smem > 48 * 1024)
-            HB2_CUDA(cudaFuncSetAttribute(k_lmg_bottom<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const size_t smem = elems * sizeof(T);      // grids of 33, 17, 9, 5 and 3 points a line: at most 36 KB
         k_lmg_bottom<T><<<1, kLBottomThreads, smem, s>>>(g);
         count_launches(1);
         HB2_LAUNCH_CHECK("lmg bottom");

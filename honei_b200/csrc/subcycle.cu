@@ -423,13 +423,16 @@ namespace hb2
     }
 
     // widest cluster (16 CTAs of 1024 threads, else 8) that can be resident,
-    // per kernel, computed once outside any stream capture (subcycle_prepare)
+    // per kernel and device, computed once outside any stream capture (subcycle_prepare)
     static int cluster_width(const void * fn, int threads = 1024)
     {
         static std::mutex mu;
-        static std::map<const void *, int> widths;
+        static std::map<std::pair<const void *, int>, int> widths;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const auto key = std::make_pair(fn, dev);
         std::lock_guard<std::mutex> lock(mu);
-        auto it = widths.find(fn);
+        auto it = widths.find(key);
         if (it != widths.end()) return it->second;
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         int width = 1;
@@ -457,7 +460,7 @@ namespace hb2
             }
             cudaGetLastError();
         }
-        widths[fn] = width;
+        widths[key] = width;
         return width;
     }
 
