@@ -477,7 +477,10 @@ extern "C" int hb2_cg_solve(hb2_ell A, const void * b, void * x, uint64_t max_it
     HB2_CUDA(cudaMemsetAsync(ws->scalars + 8, 0, 2 * sizeof(double), stream));
     const size_t es = dtype_size(A->dtype), n = A->rows;
     if (n == 0) { if (used_iters) *used_iters = 0; if (final_defect) *final_defect = 0; return HB2_OK; }
-    // a Q1 grid operator that fits a cluster; otherwise one block, or the whole GPU
+    // a Q1 grid operator that fits a cluster; otherwise one block, or the whole GPU, whose grid
+    // barrier is the only bounded wait: the other forms neither set nor read the error word
+    // (another call's expired wait on this stream may have left it set)
+    bool whole_gpu = false;
     st = cg_cluster_applies(A) ? launch_cg_cluster(A, b, x, max_iters, eps, used_dev, def_dev, stream)
                                : HB2_ERR_UNSUPPORTED;
     if (st == HB2_OK) {}
@@ -488,6 +491,7 @@ extern "C" int hb2_cg_solve(hb2_ell A, const void * b, void * x, uint64_t max_it
     }
     else
     {
+        whole_gpu = true;
         void * tmp = 0;
         const size_t vb = (n * es + 255) / 256 * 256;   // each vector 256-byte aligned
         HB2_CUDA(cudaMallocAsync(&tmp, 3 * vb + 64, stream));
@@ -527,9 +531,9 @@ extern "C" int hb2_cg_solve(hb2_ell A, const void * b, void * x, uint64_t max_it
     }
     HB2_CUDA(cudaMemcpyAsync(ws->host_scalars, ws->scalars + 8, 2 * sizeof(double), cudaMemcpyDeviceToHost, stream));
     int herr = 0;
-    HB2_CUDA(cudaMemcpyAsync(ws->host_scalars + 2, ws->error, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    if (whole_gpu) HB2_CUDA(cudaMemcpyAsync(ws->host_scalars + 2, ws->error, sizeof(int), cudaMemcpyDeviceToHost, stream));
     HB2_CUDA(cudaStreamSynchronize(stream));
-    memcpy(&herr, ws->host_scalars + 2, sizeof(int));
+    if (whole_gpu) memcpy(&herr, ws->host_scalars + 2, sizeof(int));
     if (herr) return fail(HB2_ERR_TIMEOUT, "hb2_cg_solve: a grid barrier wait expired");
     uint64_t used = 0;
     memcpy(&used, ws->host_scalars, sizeof(uint64_t));

@@ -132,3 +132,12 @@ extern "C" uint64_t hb2_workspace_count(void)
     std::lock_guard<std::mutex> lock(hb2::g_ws_mutex);
     return hb2::g_ws.size();
 }
+
+extern "C" int hb2_workspace_error(cudaStream_t stream, int ** word)
+{
+    if (! word) return hb2::fail(HB2_ERR_ARG, "hb2_workspace_error: null argument");
+    hb2::Workspace * ws = 0;
+    const int st = hb2::stream_workspace(stream, &ws);
+    if (! st) *word = ws->error;
+    return st;
+}

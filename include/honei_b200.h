@@ -79,6 +79,9 @@ HB2_API uint64_t hb2_launch_count(void);
  * allocated since load (each is created on the first fused reduction on a
  * stream and kept until exit) */
 HB2_API uint64_t hb2_workspace_count(void);
+/* device address of the word of `stream`'s workspace in which a bounded device-side wait
+ * that expired leaves a 1 (HB2_ERR_TIMEOUT); for tests, which preset it */
+HB2_API int hb2_workspace_error(cudaStream_t stream, int **word);
 
 /* ---------------------------------------------------------------- matrices */
 /* Upload a SparseMatrixELL in the reference layout (la/sparse_matrix_ell-impl.hh:42-72:

@@ -3,11 +3,14 @@ operator as one cluster (csrc/cg_cluster.cu, math/cg.hh:64-135) and CGSolver VAR
 vector P as one cooperative launch (csrc/krylov.cu, math/cg.hh:142-210), at the sizes
 where their splits change.  The dots are summed in another order than the reference's, so
 a solve may stop a step earlier or later and is held to its own stopping test."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 import honei_b200 as hb
+from honei_b200 import _lib
 from honei_b200 import DenseVector, SparseMatrixELL
 from honei_b200.inputs import q1_coefficient_operator, uniform
 
@@ -62,6 +65,29 @@ def test_cluster_cg_f32():
     hb.Defect.value(r, b, A, x)
     # 1e-4 by the recursion, 1e-4 again for its drift over some 200 steps of 6e-8
     assert hb.Norm.value(r) < 2e-4 * hb.Norm.value(b)
+
+
+# one warp, one CTA, a cluster, and the whole GPU with its grid barrier, which clears the word
+@pytest.mark.parametrize("level", [3, 5, 7, 9])
+def test_an_expired_wait_of_another_call_is_not_this_solve_s(level):
+    """A 1 left in the stream's error word (here from the host) says nothing about a later solve."""
+    word = ctypes.c_void_p()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert _lib.load().hb2_workspace_error(stream, ctypes.byref(word)) == 0
+
+    class Word:
+        __cuda_array_interface__ = {"shape": (1,), "typestr": "<i4", "data": (word.value, False), "version": 2}
+    flag = torch.as_tensor(Word(), device="cuda")
+    A = SparseMatrixELL.poisson_q1(level)
+    b = dvec(uniform(A.rows(), 3))
+    x, y = dvec(np.zeros(A.rows())), dvec(np.zeros(A.rows()))
+    used = hb.CGSolver.value(A, None, b, x, 30, 1e-8)[1]
+    flag.fill_(1)
+    try:
+        assert hb.CGSolver.value(A, None, b, y, 30, 1e-8)[1] == used
+    finally:
+        flag.zero_()
+    assert np.array_equal(x.numpy().view(np.uint8), y.numpy().view(np.uint8))
 
 
 # rows a thread: 1 (one block of 5), 1, 2 and 3
