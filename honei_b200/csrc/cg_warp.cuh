@@ -36,15 +36,17 @@ namespace hb2
     // groups of four lanes, each lane receives two neighbouring groups' sums and adds them,
     // and S(8x4) * ones(4x8) sums those four values.  Measured (B200): 66 cycles against 176
     // (a 64-bit shuffle and its add take 35, a product 29).  Every product is by one, so the
-    // result is a sum of the 32 values in a fixed order.
+    // result is a sum of the 32 values in a fixed order.  Volatile: every lane has to take part
+    // where the call stands, so the compiler must not sink it into a branch that alone uses the
+    // result (the callers' "if (lane == 0) ... = sum").
     __device__ __forceinline__ double warp_sum_mma(double v)
     {
         double d0, d1, e0, e1;
         const double one = 1.0, zero = 0.0;
-        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
                      : "=d"(d0), "=d"(d1) : "d"(one), "d"(v), "d"(zero), "d"(zero));
         const double s = d0 + d1;
-        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
                      : "=d"(e0), "=d"(e1) : "d"(s), "d"(one), "d"(zero), "d"(zero));
         return e0;
     }
