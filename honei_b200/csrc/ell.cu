@@ -411,7 +411,8 @@ namespace hb2
         size_t vbytes = nslots * dtype_size(dtype), cbytes = nslots * sizeof(int32_t);
         cudaError_t e = cudaMalloc(&A->val, std::max<size_t>(vbytes, 16));
         if (e != cudaSuccess) { delete A; return cuda_status(e, "ELL values cudaMalloc"); }
-        e = cudaMalloc(&A->col, std::max<size_t>(cbytes, 16));
+        // behind the indices, the scratch of the row check at creation (ell_find_q1_grid)
+        e = cudaMalloc(&A->col, cbytes + kEllScratchBytes);
         if (e != cudaSuccess) { cudaFree(A->val); delete A; return cuda_status(e, "ELL indices cudaMalloc"); }
         A->bytes = vbytes + cbytes;
         *out = A;

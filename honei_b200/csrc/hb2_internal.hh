@@ -343,6 +343,9 @@ namespace hb2
     int launch_grid9(const hb2_ell_s * A, int mode, const void * x, void * y, const void * aux, const void * aux2,
                      double * red, int want_sqrt, const Workspace * ws, cudaStream_t stream, int flags);
     bool q1_transfer_kernels_enabled();   // HB2_Q1_TRANSFER=0 turns them off (ell.cu)
+    // after the indices of a matrix (col + K * ld): room of its own for the check's reference row
+    // and flag, so that matrices may be made from several threads on one stream
+    constexpr size_t kEllScratchBytes = 128;
     int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream);
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);
     // one product, defect or product with dot (kPlain, kDefect, kDot) as a streaming pass; the

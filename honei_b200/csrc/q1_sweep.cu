@@ -45,13 +45,12 @@ namespace hb2
     static int find_grid_typed(hb2_ell_s * A, uint32_t m, cudaStream_t stream)
     {
         const EllView<T> V = A->view<T>();
-        // the stream's workspace holds the row and the flag (no allocation, no device-wide wait)
-        Workspace * ws = 0;
-        int st = stream_workspace(stream, &ws);
-        if (st) return st;
+        // the row and the flag in the matrix's own scratch: a place shared by the stream's calls would
+        // mix up two matrices that two threads make at the same time
         T ref[10];
-        T * dref = (T *)(ws->scalars + 32);
-        int * dbad = (int *)(ws->scalars + 44);
+        T * dref = (T *)(A->col + (uint64_t)A->K * A->ld);
+        int * dbad = (int *)(dref + 10);
+        static_assert(10 * sizeof(T) + sizeof(int) <= kEllScratchBytes, "reference row and flag");
         HB2_CUDA(cudaMemsetAsync(dbad, 0, sizeof(int), stream));
         HB2_CUDA(cudaMemcpy2DAsync(dref, sizeof(T), V.val + m + 1, V.ld * sizeof(T), sizeof(T), 9,
                                    cudaMemcpyDeviceToDevice, stream));

@@ -116,3 +116,27 @@ def test_two_krylov_solvers_of_one_instance(order):
         x = s[0].solve(s[1], dvec(np.zeros(s[2])))[0].numpy()
         if s is first:
             assert np.array_equal(x.view(np.uint8), alone.view(np.uint8))
+
+
+def test_matrices_made_on_one_stream():
+    """Two threads make a constant-coefficient grid operator and a varying one, again and again,
+    on the same stream: each keeps its own rows (one was taken for the other now and then when
+    the check of the rows kept its reference row in the stream's workspace)."""
+    cells = 6
+    n = (cells + 1) ** 2
+    ops = [q1_coefficient_operator(np.ones((cells, cells))),
+           q1_coefficient_operator(np.power(4.0, uniform(cells * cells, 5, -0.5, 0.5)).reshape(cells, cells))]
+    x = dvec(uniform(n, 3))
+    b, P = dvec(uniform(n, 4)), dvec(np.full(n, 0.25))
+    stream = torch.cuda.current_stream()
+
+    def smooth(A):
+        y, t = x.copy(), dvec(np.zeros(n))
+        return hb.RISmoother.value(A, P, b, y, temps=[t], max_iters=3).elements
+    alone = [smooth(SparseMatrixELL.from_arrays(*op)).cpu() for op in ops]
+
+    def make(k, count=1500):
+        return [SparseMatrixELL.from_arrays(*ops[k], stream=stream) for _ in range(count)]
+    for k, made in enumerate(in_threads(lambda: make(0), lambda: make(1))):
+        for A in made:
+            assert torch.equal(smooth(A).cpu(), alone[k])
