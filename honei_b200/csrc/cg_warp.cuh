@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cfloat>
+#include <type_traits>
 
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
@@ -49,6 +50,22 @@ namespace hb2
         asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %5};"
                      : "=d"(e0), "=d"(e1) : "d"(s), "d"(one), "d"(zero), "d"(zero));
         return e0;
+    }
+
+    // the same for two values, whose instructions overlap (volatile ones keep their order)
+    __device__ __forceinline__ void warp_sum_mma2(double & a, double & b)
+    {
+        double a0, a1, b0, b1;
+        const double one = 1.0, zero = 0.0;
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%4}, {%5}, {%7, %7};\n\t"
+                     "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%2, %3}, {%4}, {%6}, {%7, %7};"
+                     : "=&d"(a0), "=&d"(a1), "=&d"(b0), "=&d"(b1) : "d"(one), "d"(a), "d"(b), "d"(zero));
+        const double s = a0 + a1, t = b0 + b1;
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%4}, {%6}, {%7, %7};\n\t"
+                     "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%2, %3}, {%5}, {%6}, {%7, %7};"
+                     : "=&d"(a0), "=&d"(a1), "=&d"(b0), "=&d"(b1) : "d"(s), "d"(t), "d"(one), "d"(zero));
+        a = a0;
+        b = b0;
     }
 
     // ------------------------------------------------------------------ one warp
@@ -108,7 +125,7 @@ namespace hb2
         // the gathers of the old one before the writes of the new one
         T * sp = smem;
         T * sp2 = sp + n + 1;
-        T * sa = sp + n + 1;      // first dot operand (exact mode)
+        T * sa = sp + n;          // first dot operand (exact mode, which has no such zero)
         T * sb = sa + n;          // second dot operand (exact mode)
         T av[RPL][K];
         int ac[RPL][K];
@@ -140,9 +157,10 @@ namespace hb2
                 out[j] = s;
             }
         };
-        // dot of per-lane register vectors a, b over the valid rows
-        auto dot = [&](const T (&a)[RPL], const T (&bb)[RPL]) -> T {
-            if (exact == kCgExact)
+        // dot of per-lane register vectors a, b over the valid rows; `order` is a constant, so that
+        // neither mode's loop carries the other's instructions
+        auto dot = [&](const T (&a)[RPL], const T (&bb)[RPL], auto order) -> T {
+            if constexpr (decltype(order)::value)
             {
 #pragma unroll
                 for (int j = 0; j < RPL; ++j)
@@ -191,7 +209,7 @@ namespace hb2
         if (exact != kCgExact && lane == 0) sp[n] = sp2[n] = T(0);     // (the exact mode's dots use this memory)
         __syncwarp();
         const T eps = T(eps_d);
-        T alpha = dot(rr, rr);
+        T alpha = exact == kCgExact ? dot(rr, rr, std::true_type()) : dot(rr, rr, std::false_type());
         const T initial = sqrt(alpha);
         T current = initial;
         uint64_t it = 0, used = 0;
@@ -273,43 +291,48 @@ namespace hb2
             }
             it = max_iters;   // done: skip the loop below
         }
-        while (it < max_iters)
-        {
-            // the tree-ordered mode takes the fused product and reciprocals, that of the old
-            // alpha while the product's dot is on its way
-            T inv_alpha = T(0);
-            if (exact == kCgExact) spmv(vr);
-            else
+        auto standard = [&](auto order) {
+            constexpr bool EXACT = decltype(order)::value;
+            while (it < max_iters)
             {
-                spmv_tree(vr, sp);
-                inv_alpha = Recip<T>::rn(guard(alpha));
-            }
-            const T temp = dot(vr, pr);
-            const T lambda = exact == kCgExact ? M::div(alpha, guard(temp)) : M::mul(alpha, Recip<T>::rn(guard(temp)));
-            const T mlambda = -lambda;
+                // the tree-ordered mode takes the fused product and reciprocals, that of the old
+                // alpha while the product's dot is on its way
+                T inv_alpha = T(0);
+                if constexpr (EXACT) spmv(vr);
+                else
+                {
+                    spmv_tree(vr, sp);
+                    inv_alpha = Recip<T>::rn(guard(alpha));
+                }
+                const T temp = dot(vr, pr, order);
+                const T lambda = EXACT ? M::div(alpha, guard(temp)) : M::mul(alpha, Recip<T>::rn(guard(temp)));
+                const T mlambda = -lambda;
 #pragma unroll
-            for (int j = 0; j < RPL; ++j)
-            {
-                xr[j] = M::add(xr[j], M::mul(lambda, pr[j]));
-                rr[j] = M::add(rr[j], M::mul(mlambda, vr[j]));
-            }
-            const T alpha_old = alpha;
-            alpha = dot(rr, rr);
-            const T talpha = exact == kCgExact ? M::div(alpha, guard(alpha_old)) : M::mul(alpha, inv_alpha);
-            __syncwarp();   // every lane is done gathering the old p
+                for (int j = 0; j < RPL; ++j)
+                {
+                    xr[j] = M::add(xr[j], M::mul(lambda, pr[j]));
+                    rr[j] = M::add(rr[j], M::mul(mlambda, vr[j]));
+                }
+                const T alpha_old = alpha;
+                alpha = dot(rr, rr, order);
+                const T talpha = EXACT ? M::div(alpha, guard(alpha_old)) : M::mul(alpha, inv_alpha);
+                __syncwarp();   // every lane is done gathering the old p
 #pragma unroll
-            for (int j = 0; j < RPL; ++j)
-            {
-                const int row = lane + 32 * j;
-                pr[j] = M::add(M::mul(pr[j], talpha), rr[j]);
-                if (row < n) sp[row] = pr[j];
+                for (int j = 0; j < RPL; ++j)
+                {
+                    const int row = lane + 32 * j;
+                    pr[j] = M::add(M::mul(pr[j], talpha), rr[j]);
+                    if (row < n) sp[row] = pr[j];
+                }
+                __syncwarp();
+                ++it;
+                current = sqrt(alpha);
+                if (current < M::mul(eps, initial) || current < eps) { used = it; break; }
+                if (it == max_iters) used = it;
             }
-            __syncwarp();
-            ++it;
-            current = sqrt(alpha);
-            if (current < M::mul(eps, initial) || current < eps) { used = it; break; }
-            if (it == max_iters) used = it;
-        }
+        };
+        if (exact == kCgExact) standard(std::true_type());
+        else standard(std::false_type());
 #pragma unroll
         for (int j = 0; j < RPL; ++j)
             if (lane + 32 * j < n) xg[lane + 32 * j] = S(xr[j]);

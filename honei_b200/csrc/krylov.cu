@@ -301,8 +301,8 @@ namespace
         // the next ones while another still reads these)
         auto total = [&](double & a0, double & a1, bool two) -> bool {
             double * part = g.partials + (two ? gridDim.x : 0);
-            a0 = warp_sum_mma(a0);
-            if (two) a1 = warp_sum_mma(a1);
+            if (two) warp_sum_mma2(a0, a1);
+            else a0 = warp_sum_mma(a0);
             if (lane == 0)
             {
                 wred[0][warp] = a0;
@@ -311,8 +311,10 @@ namespace
             __syncthreads();
             if (warp == 0)
             {
-                const double s0 = warp_sum_mma(lane < kLoopThreads / 32 ? wred[0][lane] : 0.0);
-                const double s1 = two ? warp_sum_mma(lane < kLoopThreads / 32 ? wred[1][lane] : 0.0) : 0.0;
+                double s0 = lane < kLoopThreads / 32 ? wred[0][lane] : 0.0;
+                double s1 = two && lane < kLoopThreads / 32 ? wred[1][lane] : 0.0;
+                if (two) warp_sum_mma2(s0, s1);
+                else s0 = warp_sum_mma(s0);
                 if (lane == 0)
                 {
                     part[blockIdx.x] = s0;
@@ -327,8 +329,10 @@ namespace
                 s0 += __ldcg(part + b);
                 if (two) s1 += __ldcg(part + gridDim.x + b);
             }
-            a0 = warp_sum_mma(s0);
-            if (two) a1 = warp_sum_mma(s1);
+            if (two) warp_sum_mma2(s0, s1);
+            else s0 = warp_sum_mma(s0);
+            a0 = s0;
+            a1 = s1;
             return true;
         };
         while (true)
