@@ -227,12 +227,19 @@ namespace
         if (ok) xout[i] = x;
     }
 
+    // two kernels: in one, the thread form lost 9 % in FP32 (81 unknowns) to the warp form beside it
     template <typename T>
     __global__ void k_coarse_cg(const T * bands, uint64_t n, uint64_t m, const T * rhs, T * x, T * g, T * u, T * e,
                                 T * ng, double konv_rad, uint64_t cap, LState * st)
     {
-        if (n <= 32) coarse_cg_warp(bands, (int)n, (int)m, rhs, x, konv_rad, cap, st);
-        else if (threadIdx.x == 0) coarse_cg_thread(bands, n, m, rhs, x, g, u, e, ng, konv_rad, cap, st);
+        coarse_cg_thread(bands, n, m, rhs, x, g, u, e, ng, konv_rad, cap, st);
+    }
+
+    template <typename T>
+    __global__ void __launch_bounds__(32) k_coarse_cg_warp(const T * bands, int n, int m, const T * rhs, T * x, double konv_rad,
+                                                           uint64_t cap, LState * st)
+    {
+        coarse_cg_warp(bands, n, m, rhs, x, konv_rad, cap, st);
     }
 
     // out = x + alpha P c in one pass (the prolonged correction, math/prolongation.hh, then
@@ -461,6 +468,24 @@ namespace
         return t;
     }
 
+    // the coarsest level's solve of A x = rhs, a launch of its own
+    template <typename T>
+    int launch_coarse(hb2_lmg_s * G, const void * rhs, cudaStream_t s)
+    {
+        auto & C = G->lev[0];
+        const double konv_rad = (double)std::numeric_limits<T>::epsilon();
+        const T * bands = (const T *)C.A->bands;
+        T * g = (T *)G->cg;
+        if (C.n <= 32)
+            k_coarse_cg_warp<T><<<1, 32, 0, s>>>(bands, (int)C.n, (int)C.m, (const T *)rhs, (T *)C.x, konv_rad, 100000, G->st);
+        else
+            k_coarse_cg<T><<<1, 1, 0, s>>>(bands, C.n, C.m, (const T *)rhs, (T *)C.x, g, g + C.n, g + 2 * C.n, g + 3 * C.n,
+                                           konv_rad, 100000, G->st);
+        count_launches(1);
+        HB2_LAUNCH_CHECK("lmg coarse cg");
+        return HB2_OK;
+    }
+
     template <typename T>
     int launch_bottom(hb2_lmg_s * G, int top, cudaStream_t s)
     {
@@ -498,16 +523,11 @@ namespace
         const uint64_t npre = G->prm.n_pre_smooth;
         const T alpha = (T)G->prm.adapt_correction_factor;
         auto & C = G->lev[0];
-        T * cgv = (T *)G->cg;
-        const uint64_t nc = C.n;
         int st = HB2_OK;
         if (nl == 1)
         {
-            k_coarse_cg<T><<<1, 32, 0, s>>>((const T *)C.A->bands, C.n, C.m, (const T *)C.d, (T *)C.x, cgv, cgv + nc,
-                                           cgv + 2 * nc, cgv + 3 * nc, (double)std::numeric_limits<T>::epsilon(),
-                                           100000, G->st);
-            count_launches(1);
-            HB2_LAUNCH_CHECK("lmg coarse cg");
+            st = launch_coarse<T>(G, C.d, s);
+            if (st) return st;
             return launch_q1(C.A, 1, C.x, C.d, C.rhs, nullptr, G->ws->error, s);
         }
         const int bottom = bottom_top(G);
@@ -541,14 +561,7 @@ namespace
         }
         if (st) return st;
         if (bottom > 0) st = launch_bottom<T>(G, bottom, s);
-        else
-        {
-            k_coarse_cg<T><<<1, 32, 0, s>>>((const T *)C.A->bands, C.n, C.m, (const T *)C.rhs, (T *)C.x, cgv, cgv + nc,
-                                            cgv + 2 * nc, cgv + 3 * nc, (double)std::numeric_limits<T>::epsilon(),
-                                            100000, G->st);
-            count_launches(1);
-            HB2_LAUNCH_CHECK("lmg coarse cg");
-        }
+        else st = launch_coarse<T>(G, C.rhs, s);
         if (st) return st;
         for (unsigned i = (unsigned)bottom + 1; i < nl && ! st; ++i)
         {
