@@ -76,6 +76,7 @@ struct hb2_csr_s
     uint2 * xwin = nullptr;
     uint32_t nwindows = 0, win_bytes = 0;
     bool staged = false;
+    bool deep = false;             // long rows: each task in a CTA of its own (run_long_deep)
     // long rows
     uint4 * items = nullptr;       // (row | flags, 0, first entry, end entry)
     uint32_t * tasks = nullptr;    // nlong_warps + 1 item offsets
@@ -510,9 +511,7 @@ namespace
     template <typename T, bool DEFECT>
     int launch(hb2_csr A, const void * rhs, const void * x, void * y, cudaStream_t stream)
     {
-        // few long rows: each task in a CTA of its own, eight chunks deep;
-        // with more of them than SMs the four-warp form keeps more chains resident
-        const int deep = A->nlong_warps <= (uint32_t)num_sms();
+        const bool deep = A->deep;
         const uint32_t long_ctas = deep ? A->nlong_warps : (A->nlong_warps + kCsrWarps - 1) / kCsrWarps;
         const uint32_t slice_ctas = (A->nslices + kCsrWarps - 1) / kCsrWarps;
         if (long_ctas + slice_ctas == 0) return HB2_OK;
@@ -542,9 +541,9 @@ namespace
         return HB2_OK;
     }
 
-    // Slots loaded per lane and round in the sliced part, 8 or 16, and x gathered from
-    // global memory or staged by window: whichever runs the product fastest on this
-    // matrix (timed at creation when it holds at least 2^18 slots; bit-identical
+    // Slots loaded per lane and round in the sliced part, 8 or 16, x gathered from
+    // global memory or staged by window, and few long rows in CTAs of their own or four to
+    // one: whichever runs the product fastest on this matrix (timed at creation when it holds at least 2^18 slots; bit-identical
     // results either way).  Measured on the
     // level-11 Q1 operator: FP64 108.6 us (16) / 127.0 us (8), FP32 83.9 us (16)
     // / 75.0 us (8).  HB2_CSR_U=8|16 fixes it.
@@ -553,11 +552,17 @@ namespace
     {
         A->unroll = 8;
         A->staged = false;
+        // few long rows: each task in a CTA of its own, eight chunks deep; with more of them than
+        // SMs the four-warp form keeps more chains resident
+        const bool few = A->nlong_warps <= (uint32_t)num_sms();
+        A->deep = few;
         if (const char * env = getenv("HB2_CSR_U"))
         {
             A->unroll = atoi(env) == 16 ? 16 : 8;
             const char * st = getenv("HB2_CSR_STAGED");     // with HB2_CSR_U: 1 stages x where it fits
             A->staged = st && atoi(st) == 1 && A->win_bytes;
+            const char * dp = getenv("HB2_CSR_DEEP");       // with HB2_CSR_U: 0 runs few long rows four to a CTA too
+            A->deep = few && (A->staged || ! (dp && atoi(dp) == 0));
             return HB2_OK;
         }
         if (A->nslots + A->nlong_entries < (1u << 18)) return HB2_OK;
@@ -568,28 +573,31 @@ namespace
         cudaEvent_t ev[2] = {nullptr, nullptr};
         if (e == cudaSuccess) e = cudaEventCreate(&ev[0]);
         if (e == cudaSuccess) e = cudaEventCreate(&ev[1]);
-        float best = 1e30f;
-        int best_u = 8;
-        bool best_staged = false;
-        for (int v = 0; v < (A->win_bytes ? 4 : 2); ++v)
+        // the deep form's buffers (24 KB a CTA in FP64) leave the slices fewer warps an SM, which
+        // costs more than the long rows' chains where the slices gather over all of x (60,000 rows,
+        // columns anywhere, 16 long rows, FP64: 42.7 us deep, 33.1 shared): both are timed
+        struct Form { int unroll; bool staged, deep; };
+        std::vector<Form> forms = {{8, false, few}, {16, false, few}};
+        if (A->win_bytes) { forms.push_back({8, true, few}); forms.push_back({16, true, few}); }
+        if (few && A->nlong_warps) { forms.push_back({8, false, false}); forms.push_back({16, false, false}); }
+        auto select = [&](const Form & f) {
+            A->unroll = f.unroll;
+            A->staged = f.staged;
+            A->deep = f.deep;
+        };
+        std::vector<float> time(forms.size(), 1e30f);
+        for (size_t v = 0; v < forms.size() && e == cudaSuccess; ++v)
         {
-            const int u = v & 1 ? 16 : 8;
-            if (e != cudaSuccess) break;
-            A->unroll = u;
-            A->staged = v >= 2;
-            int st = launch<T, false>(A, nullptr, x, y, stream);    // warm-up
-            if (st) { e = cudaErrorUnknown; break; }
+            select(forms[v]);
+            if (launch<T, false>(A, nullptr, x, y, stream)) { e = cudaErrorUnknown; break; }    // warm-up
             e = cudaEventRecord(ev[0], stream);
             for (int i = 0; i < 3 && e == cudaSuccess; ++i)
                 if (launch<T, false>(A, nullptr, x, y, stream)) e = cudaErrorUnknown;
             if (e == cudaSuccess) e = cudaEventRecord(ev[1], stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
-            float ms = 0;
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev[0], ev[1]);
-            if (e == cudaSuccess && ms < best) { best = ms; best_u = u; best_staged = A->staged; }
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&time[v], ev[0], ev[1]);
         }
-        A->unroll = best_u;
-        A->staged = best_staged;
+        select(forms[std::min_element(time.begin(), time.end()) - time.begin()]);
         if (ev[0]) cudaEventDestroy(ev[0]);
         if (ev[1]) cudaEventDestroy(ev[1]);
         cudaFree(x);
@@ -699,32 +707,32 @@ namespace
         }
         std::vector<int32_t> scol(nslots, -1);
         std::vector<T> sval(nslots, T(0));
+        // first and last column of each window of kSigma short rows
+        const uint32_t nwindows = (uint32_t)((short_rows.size() + kSigma - 1) / kSigma);
+        std::vector<std::pair<int32_t, int32_t>> span(nwindows, std::make_pair(INT32_MAX, -1));
         for (uint64_t sl = 0; sl < nslices; ++sl)
             for (uint64_t j = 0; j < H; ++j)
             {
                 const uint32_t r = perm[H * sl + j];
                 if (r == 0xffffffffu) continue;
+                auto & sp = span[sl / kWinWarps];
                 for (uint64_t k = 0; k < len(r); ++k)
                 {
-                    scol[slices[sl].x + H * k + j] = ecol[start[r] + k];
+                    const int32_t c = ecol[start[r] + k];
+                    sp.first = std::min(sp.first, c);
+                    sp.second = std::max(sp.second, c);
+                    scol[slices[sl].x + H * k + j] = c;
                     sval[slices[sl].x + H * k + j] = eval[start[r] + k];
                 }
             }
         // each window's span of x; the staged kernel is a candidate when nine windows in ten fit
         // and the long rows are few enough for a CTA each
-        const uint32_t nwindows = (uint32_t)((short_rows.size() + kSigma - 1) / kSigma);
         std::vector<uint2> xwin(nwindows);
         uint64_t span_max = 1;
         uint32_t wide = 0;
         for (uint32_t w = 0; w < nwindows; ++w)
         {
-            int32_t lo = INT32_MAX, hi = -1;
-            for (size_t q = (size_t)w * kSigma; q < std::min<size_t>(short_rows.size(), (size_t)(w + 1) * kSigma); ++q)
-                for (uint64_t i = start[short_rows[q]]; i < start[short_rows[q] + 1]; ++i)
-                {
-                    lo = std::min(lo, ecol[i]);
-                    hi = std::max(hi, ecol[i]);
-                }
+            const int32_t lo = span[w].first, hi = span[w].second;
             xwin[w] = hi < 0 ? make_uint2(0, 0) : make_uint2((uint32_t)lo, (uint32_t)(hi - lo + 1));
             if ((uint64_t)xwin[w].y * sizeof(T) > kWinBytes)
             {
@@ -756,7 +764,7 @@ namespace
         A->nlong_entries = lcol.size();
         A->bytes = sizeof(uint2) * nslices + sizeof(uint32_t) * perm.size() + (sizeof(int32_t) + sizeof(T)) * nslots +
                    sizeof(uint4) * items.size() + sizeof(uint32_t) * tasks.size() +
-                   (sizeof(int32_t) + sizeof(T)) * lcol.size();
+                   (sizeof(int32_t) + sizeof(T)) * lcol.size() + (fits ? sizeof(uint2) * nwindows : 0);
         return HB2_OK;
     }
 }

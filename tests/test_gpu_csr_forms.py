@@ -44,3 +44,25 @@ def test_forms(oracle, monkeypatch, rows, nlong, longest, npdt, staged, u):
     assert np.array_equal(y.numpy().view(np.uint8), oracle.csr_spmv(ref, x).view(np.uint8))
     hb.Defect.value(y, DenseVector(torch.from_numpy(b).cuda()), A, xd)
     assert np.array_equal(y.numpy().view(np.uint8), oracle.csr_defect(ref, b, x).view(np.uint8))
+
+
+@pytest.mark.parametrize("npdt", [np.float64, np.float32])
+@pytest.mark.parametrize("u", ["8", "16"])
+@pytest.mark.parametrize("nlong", [1, 5])
+def test_few_long_rows_four_to_a_cta(oracle, monkeypatch, npdt, u, nlong):
+    """The form of many long rows on a few of them, chosen where the slices gather over all of x."""
+    monkeypatch.setenv("HB2_CSR_U", u)
+    monkeypatch.setenv("HB2_CSR_DEEP", "0")
+    rows = 1500
+    rng = np.random.default_rng(nlong)
+    length = rng.integers(0, 40, rows)
+    length[rng.permutation(rows)[:nlong]] = rng.integers(129, 1400, nlong)
+    ar = np.zeros(rows + 1, np.int64)
+    np.cumsum(length, out=ar[1:])
+    aj = rng.integers(0, rows, int(ar[-1]))
+    ax, x = uniform(aj.size, 3, dtype=npdt), uniform(rows, 4, dtype=npdt)
+    A = SparseMatrixCSR.from_arrays(rows, rows, ar, aj, ax)
+    y = DenseVector(rows, dtype=torch.float64 if npdt == np.float64 else torch.float32)
+    hb.Product.value(y, A, DenseVector(torch.from_numpy(x).cuda()))
+    ref = oracle.csr_spmv(oracle.csr_blocked(rows, rows, ar, aj, ax), x)
+    assert np.array_equal(y.numpy().view(np.uint8), ref.view(np.uint8))
