@@ -411,7 +411,7 @@ namespace hb2
         size_t vbytes = nslots * dtype_size(dtype), cbytes = nslots * sizeof(int32_t);
         cudaError_t e = cudaMalloc(&A->val, std::max<size_t>(vbytes, 16));
         if (e != cudaSuccess) { delete A; return cuda_status(e, "ELL values cudaMalloc"); }
-        // behind the indices, the scratch of the row check at creation (ell_find_q1_grid)
+        // behind the indices, the scratch of the creation's checks (ell_scratch)
         e = cudaMalloc(&A->col, cbytes + kEllScratchBytes);
         if (e != cudaSuccess) { cudaFree(A->val); delete A; return cuda_status(e, "ELL indices cudaMalloc"); }
         A->bytes = vbytes + cbytes;
@@ -450,8 +450,23 @@ namespace hb2
     // Q1 Poisson operator (math/fill_matrix.hh:37-79 -> SparseMatrix -> ELL):
     // 1-based row i is a Dirichlet unit row when i <= M, i > N-M, i%M == 1 or
     // i%M == 0; interior rows hold the 9 stencil entries in ascending column order.
+    template <typename T> struct Q1Row { T v[9]; };
+
     template <typename T>
-    __global__ void ell_q1_kernel(uint64_t M, double aniso, uint64_t ld, T * val, int32_t * col)
+    static Q1Row<T> q1_interior_row(double aniso)
+    {
+        Q1Row<T> q;
+        for (int k = 0; k < 9; ++k)
+        {
+            q.v[k] = T(-1.0 / 3.0);
+            if (k == 4) q.v[k] = aniso == 1.0 ? T(8.0 / 3.0) : T((6.0 + 2.0 * aniso) / 3.0);
+            else if ((k == 3 || k == 5) && aniso != 1.0) q.v[k] = T(-aniso / 3.0);
+        }
+        return q;
+    }
+
+    template <typename T>
+    __global__ void ell_q1_kernel(uint64_t M, const __grid_constant__ Q1Row<T> row, uint64_t ld, T * val, int32_t * col)
     {
         uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (r >= ld) return;
@@ -472,13 +487,9 @@ namespace hb2
         }
         const int64_t m = (int64_t)M;
         const int64_t off[9] = {-m - 1, -m, -m + 1, -1, 0, 1, m - 1, m, m + 1};
-        const T nb = T(-1.0 / 3.0);
         for (int k = 0; k < 9; ++k)
         {
-            T v = nb;
-            if (k == 4) v = aniso == 1.0 ? T(8.0 / 3.0) : T((6.0 + 2.0 * aniso) / 3.0);
-            else if ((k == 3 || k == 5) && aniso != 1.0) v = T(-aniso / 3.0);
-            val[k * ld + r] = v;
+            val[k * ld + r] = row.v[k];
             col[k * ld + r] = (int32_t)((int64_t)r + off[k]);
         }
     }
@@ -620,7 +631,7 @@ extern "C" int hb2_ell_create(hb2_ell * out, hb2_dtype dtype, uint64_t rows, uin
     const void * dAx = Ax;
     const uint64_t * dArl = Arl;
     void * tmp = 0;
-    int * bad = 0;
+    int * bad = (int *)ell_scratch(A) + kEllScratchBytes / sizeof(int) - 1;
     cudaError_t e = cudaSuccess;
     if (host_ptrs && rows > 0)
     {
@@ -640,8 +651,7 @@ extern "C" int hb2_ell_create(hb2_ell * out, hb2_dtype dtype, uint64_t rows, uin
             dArl = (const uint64_t *)(p + arl_off);
         }
     }
-    if (e == cudaSuccess) e = cudaMalloc(&bad, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ell_scratch(A), 0, kEllScratchBytes, stream);
     if (e == cudaSuccess)
     {
         unsigned grid = ceil_div(A->ld, 256);
@@ -654,19 +664,22 @@ extern "C" int hb2_ell_create(hb2_ell * out, hb2_dtype dtype, uint64_t rows, uin
         count_launches(1);
         e = cudaGetLastError();
     }
-    int hbad = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) st = launch_grid_check(A, stream);
+    alignas(16) char scratch[kEllScratchBytes] = {};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(scratch, ell_scratch(A), sizeof(scratch), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    int hbad = 0;
+    memcpy(&hbad, scratch + sizeof(scratch) - sizeof(int), sizeof(int));
     if (tmp) cudaFree(tmp);
-    if (bad) cudaFree(bad);
     if (e != cudaSuccess) { hb2_ell_destroy(A); return cuda_status(e, "hb2_ell_create"); }
+    if (st) { hb2_ell_destroy(A); return st; }
     if (hbad)
     {
         hb2_ell_destroy(A);
         return fail(HB2_ERR_ARG, hbad == 1 ? "hb2_ell_create: Arl exceeds num_cols_per_row"
                                            : "hb2_ell_create: column index >= columns");
     }
-    int cst = ell_build_compact(A, stream);
+    int cst = ell_build_compact(A, stream, grid_check_result(A, scratch));
     if (cst) { hb2_ell_destroy(A); return cst; }
     *out = A;
     return HB2_OK;
@@ -683,12 +696,27 @@ extern "C" int hb2_ell_create_q1(hb2_ell * out, hb2_dtype dtype, unsigned level,
     A->ref_K = 9;
     A->ref_T = 1;
     unsigned grid = ceil_div(A->ld, 256);
-    if (dtype == HB2_F64) ell_q1_kernel<double><<<grid, 256, 0, stream>>>(M, aniso, A->ld, (double *)A->val, A->col);
-    else ell_q1_kernel<float><<<grid, 256, 0, stream>>>(M, aniso, A->ld, (float *)A->val, A->col);
+    // a Q1 grid operator by construction: its rows need no check (and no wait for one)
+    EllGrid known;
+    known.m = (uint32_t)M;
+    known.q1 = true;
+    known.row[9] = 1.0;
+    if (dtype == HB2_F64)
+    {
+        const Q1Row<double> row = q1_interior_row<double>(aniso);
+        for (int k = 0; k < 9; ++k) known.row[k] = row.v[k];
+        ell_q1_kernel<double><<<grid, 256, 0, stream>>>(M, row, A->ld, (double *)A->val, A->col);
+    }
+    else
+    {
+        const Q1Row<float> row = q1_interior_row<float>(aniso);
+        for (int k = 0; k < 9; ++k) known.row[k] = row.v[k];
+        ell_q1_kernel<float><<<grid, 256, 0, stream>>>(M, row, A->ld, (float *)A->val, A->col);
+    }
     count_launches(1);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { hb2_ell_destroy(A); return cuda_status(e, "hb2_ell_create_q1"); }
-    int cst = ell_build_compact(A, stream);
+    int cst = ell_build_compact(A, stream, known);
     if (cst) { hb2_ell_destroy(A); return cst; }
     *out = A;
     return HB2_OK;
@@ -723,13 +751,26 @@ extern "C" int hb2_ell_create_transfer(hb2_ell * prol, hb2_ell * res, hb2_dtype 
     count_launches(2);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { hb2_ell_destroy(P); hb2_ell_destroy(R); return cuda_status(e, "hb2_ell_create_transfer"); }
-    int cst = ell_build_compact(P, stream);
-    if (! cst) cst = ell_build_compact(R, stream);
+    int cst = ell_build_compact(P, stream, EllGrid());
+    if (! cst) cst = ell_build_compact(R, stream, EllGrid());
     if (cst) { hb2_ell_destroy(P); hb2_ell_destroy(R); return cst; }
     P->q1_transfer = (int)fine_level;
     R->q1_transfer = -(int)fine_level;
     *prol = P;
     *res = R;
+    return HB2_OK;
+}
+
+// the rows of a matrix that is complete on `stream`
+static int check_grid(hb2_ell_s * A, cudaStream_t stream, EllGrid * out)
+{
+    alignas(16) char scratch[kEllScratchBytes] = {};
+    HB2_CUDA(cudaMemsetAsync(ell_scratch(A), 0, sizeof(scratch), stream));
+    const int st = launch_grid_check(A, stream);
+    if (st) return st;
+    HB2_CUDA(cudaMemcpyAsync(scratch, ell_scratch(A), sizeof(scratch), cudaMemcpyDeviceToHost, stream));
+    HB2_CUDA(cudaStreamSynchronize(stream));
+    *out = grid_check_result(A, scratch);
     return HB2_OK;
 }
 
@@ -754,7 +795,22 @@ extern "C" int hb2_ell_convert(hb2_ell * out, hb2_ell src, hb2_dtype dtype, cuda
     cudaError_t e = cudaMemcpyAsync(A->col, src->col, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { hb2_ell_destroy(A); return cuda_status(e, "hb2_ell_convert"); }
-    int cst = ell_build_compact(A, stream);
+    // a Q1 grid operator stays one, with the converted values; any other matrix is checked (rounding
+    // may have made its values equal)
+    EllGrid grid_rows;
+    int cst = HB2_OK;
+    if (src->q1g_m)
+    {
+        grid_rows.m = src->q1g_m;
+        grid_rows.q1 = true;
+        for (int k = 0; k < 10; ++k)
+        {
+            const double v = k < 9 ? src->q1g_v[k] : src->q1g_vb;
+            grid_rows.row[k] = dtype == HB2_F64 ? v : (double)(float)v;
+        }
+    }
+    else cst = check_grid(A, stream, &grid_rows);
+    if (! cst) cst = ell_build_compact(A, stream, grid_rows);
     if (cst) { hb2_ell_destroy(A); return cst; }
     *out = A;
     return HB2_OK;

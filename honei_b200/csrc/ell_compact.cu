@@ -783,13 +783,21 @@ namespace hb2
         return autotune(A, stream);
     }
 
-    int ell_build_compact(hb2_ell_s * A, cudaStream_t stream)
+    int ell_build_compact(hb2_ell_s * A, cudaStream_t stream, const EllGrid & grid)
     {
         const int st = build_layouts(A, stream);
         if (st) return st;
         // a pinned layout (HB2_ELL_COMPACT) runs everywhere, sweeps included
         const char * pin = getenv("HB2_ELL_COMPACT");
-        return pin && *pin ? HB2_OK : ell_find_q1_grid(A, stream);
+        if (pin && *pin) return HB2_OK;
+        if (! grid.q1) A->g9_m = grid.m;
+        else
+        {
+            A->q1g_m = grid.m;
+            for (int k = 0; k < 9; ++k) A->q1g_v[k] = grid.row[k];
+            A->q1g_vb = grid.row[9];
+        }
+        return HB2_OK;
     }
 
     void ell_free_compact(hb2_ell_s * A)

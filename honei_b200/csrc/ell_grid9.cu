@@ -1,7 +1,7 @@
 // ELL matrices with the rows of a nine-point operator on an m x m grid and any values: an
 // interior row's columns are i - m - 1 .. i + m + 1 in ascending slot order, a boundary row
 // holds its diagonal in slot 0 (the Q1 finite-element operator with varying coefficients;
-// checked row by row at creation, ell_find_q1_grid).  Their columns need not be read: a row
+// checked row by row at creation, launch_grid_check).  Their columns need not be read: a row
 // moves 72 instead of 108 bytes of matrix in FP64, 36 instead of 72 in FP32.
 //
 // A thread takes 16 bytes of consecutive rows (two in FP64, four in FP32): nine 128-bit value

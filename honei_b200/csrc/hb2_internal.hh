@@ -135,7 +135,7 @@ struct hb2_ell_s
     int q1_transfer = 0;
     // points per line when every row is one of the two rows of a Q1 grid operator
     // (interior rows the nine values q1g_v, boundary rows the diagonal q1g_vb;
-    // checked row by row at creation, ell_find_q1_grid), 0 otherwise: several Jacobi
+    // checked row by row at creation, launch_grid_check), 0 otherwise: several Jacobi
     // sweeps and the transfers around them run as one pass (launch_q1_sweep)
     uint32_t q1g_m = 0;
     double q1g_v[9] = {};
@@ -300,7 +300,23 @@ namespace hb2
                                cudaStream_t stream, int flags, int R, unsigned bs);
 
     // compressed ELL layout (ell_compact.cu)
-    int ell_build_compact(hb2_ell_s * A, cudaStream_t stream);
+    // what the rows of a square matrix are: m != 0: those of a nine-point operator on an m x m grid,
+    // with q1 all interior rows the values row[0 .. 8] and all boundary rows the diagonal row[9]
+    struct EllGrid
+    {
+        uint32_t m = 0;
+        bool q1 = false;
+        double row[10] = {};
+    };
+    int ell_build_compact(hb2_ell_s * A, cudaStream_t stream, const EllGrid & grid);
+    // the check of the rows (q1_sweep.cu) into the matrix's scratch, which the caller has cleared,
+    // and its result from a copy of that scratch.  The scratch lies behind the matrix's column
+    // indices: a place shared by a stream's calls would mix up two matrices that two threads make
+    // at the same time.  Its last int is hb2_ell_create's own flag.
+    constexpr size_t kEllScratchBytes = 128;
+    inline void * ell_scratch(const hb2_ell_s * A) { return A->col + (uint64_t)A->K * A->ld; }
+    int launch_grid_check(hb2_ell_s * A, cudaStream_t stream);
+    EllGrid grid_check_result(const hb2_ell_s * A, const void * scratch);
     void ell_free_compact(hb2_ell_s * A);
     void launch_ell_compact(const hb2_ell_s * A, int mode, const void * x, void * y, const void * aux,
                             const void * aux2, void * zero, double * red, int want_sqrt, ReduceSlot rs, dim3 grid,
@@ -343,10 +359,6 @@ namespace hb2
     int launch_grid9(const hb2_ell_s * A, int mode, const void * x, void * y, const void * aux, const void * aux2,
                      double * red, int want_sqrt, const Workspace * ws, cudaStream_t stream, int flags);
     bool q1_transfer_kernels_enabled();   // HB2_Q1_TRANSFER=0 turns them off (ell.cu)
-    // after the indices of a matrix (col + K * ld): room of its own for the check's reference row
-    // and flag, so that matrices may be made from several threads on one stream
-    constexpr size_t kEllScratchBytes = 128;
-    int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream);
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);
     // one product, defect or product with dot (kPlain, kDefect, kDot) as a streaming pass; the
     // refinement's outer defect (kDefectIR)

@@ -11,13 +11,29 @@ namespace hb2
 
     // every row against the two kinds of rows of a Q1 grid operator: interior rows nine columns
     // in ascending order, boundary rows one diagonal entry in slot 0 (bad bit 0: another
-    // structure); all interior rows with the values ref[0 .. 8], all boundary rows with ref[9]
-    // (bit 1: other values)
+    // structure); all interior rows with the values of the first one, all boundary rows with those
+    // of row 0 (bit 1: other values).  ref: those ten values, for the host.
     template <typename T>
-    __global__ void q1_grid_check_kernel(EllView<T> A, uint32_t m, const T * __restrict__ ref, int * bad)
+    struct GridCheck
+    {
+        T ref[10];
+        int bad;
+    };
+
+    template <typename T>
+    __global__ void q1_grid_check_kernel(EllView<T> A, uint32_t m, GridCheck<T> * out)
     {
         const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (r >= A.rows) return;
+        T ref[10];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) ref[k] = __ldg(A.val + k * A.ld + m + 1);
+        ref[9] = __ldg(A.val);
+        if (r == 0)
+        {
+#pragma unroll
+            for (int k = 0; k < 10; ++k) out->ref[k] = ref[k];
+        }
         const uint32_t i = (uint32_t)r / m, j = (uint32_t)r - i * m;
         const bool bnd = i == 0 || j == 0 || i == m - 1 || j == m - 1;
         bool shape = true, same = true;
@@ -37,48 +53,50 @@ namespace hb2
                 same = same && v == ref[k];
             }
         }
-        if (! shape) atomicOr(bad, 1);
-        if (! same) atomicOr(bad, 2);
+        if (! shape) atomicOr(&out->bad, 1);
+        if (! same) atomicOr(&out->bad, 2);
     }
 
-    template <typename T>
-    static int find_grid_typed(hb2_ell_s * A, uint32_t m, cudaStream_t stream)
+    // points per line when the matrix can be a nine-point grid matrix, else 0
+    static uint32_t grid_points(const hb2_ell_s * A)
     {
-        const EllView<T> V = A->view<T>();
-        // the row and the flag in the matrix's own scratch: a place shared by the stream's calls would
-        // mix up two matrices that two threads make at the same time
-        T ref[10];
-        T * dref = (T *)(A->col + (uint64_t)A->K * A->ld);
-        int * dbad = (int *)(dref + 10);
-        static_assert(10 * sizeof(T) + sizeof(int) <= kEllScratchBytes, "reference row and flag");
-        HB2_CUDA(cudaMemsetAsync(dbad, 0, sizeof(int), stream));
-        HB2_CUDA(cudaMemcpy2DAsync(dref, sizeof(T), V.val + m + 1, V.ld * sizeof(T), sizeof(T), 9,
-                                   cudaMemcpyDeviceToDevice, stream));
-        HB2_CUDA(cudaMemcpyAsync(dref + 9, V.val, sizeof(T), cudaMemcpyDeviceToDevice, stream));
-        q1_grid_check_kernel<T><<<ceil_div(A->rows, 256), 256, 0, stream>>>(V, m, dref, dbad);
+        if (A->rows != A->cols || A->K != 9 || A->rows < 9 || A->rows >= (1ull << 31)) return 0;
+        uint64_t m = 3;
+        while (m * m < A->rows) ++m;
+        return m * m == A->rows ? (uint32_t)m : 0;
+    }
+
+    int launch_grid_check(hb2_ell_s * A, cudaStream_t stream)
+    {
+        const uint32_t m = grid_points(A);
+        if (! m) return HB2_OK;
+        const unsigned grid = ceil_div(A->rows, 256);
+        if (A->dtype == HB2_F64)
+            q1_grid_check_kernel<double><<<grid, 256, 0, stream>>>(A->view<double>(), m, (GridCheck<double> *)ell_scratch(A));
+        else q1_grid_check_kernel<float><<<grid, 256, 0, stream>>>(A->view<float>(), m, (GridCheck<float> *)ell_scratch(A));
         count_launches(1);
         HB2_LAUNCH_CHECK("Q1 grid check");
-        int bad = 1;
-        HB2_CUDA(cudaMemcpyAsync(ref, dref, sizeof(ref), cudaMemcpyDeviceToHost, stream));
-        HB2_CUDA(cudaMemcpyAsync(&bad, dbad, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        HB2_CUDA(cudaStreamSynchronize(stream));
-        if (bad == 2) A->g9_m = m;
-        if (bad) return HB2_OK;
-        for (int k = 0; k < 9; ++k) A->q1g_v[k] = (double)ref[k];
-        A->q1g_vb = (double)ref[9];
-        A->q1g_m = m;
         return HB2_OK;
     }
 
-    int ell_find_q1_grid(hb2_ell_s * A, cudaStream_t stream)
+    template <typename T>
+    static EllGrid grid_result_typed(uint32_t m, const void * scratch)
     {
-        A->q1g_m = A->g9_m = 0;
-        if (A->rows != A->cols || A->K != 9 || A->rows < 9 || A->rows >= (1ull << 31)) return HB2_OK;
-        uint64_t m = 3;
-        while (m * m < A->rows) ++m;
-        if (m * m != A->rows) return HB2_OK;
-        return A->dtype == HB2_F64 ? find_grid_typed<double>(A, (uint32_t)m, stream)
-                                   : find_grid_typed<float>(A, (uint32_t)m, stream);
+        const GridCheck<T> & h = *(const GridCheck<T> *)scratch;
+        static_assert(sizeof(h) <= kEllScratchBytes - sizeof(int), "scratch of the row check");
+        EllGrid g;
+        if (h.bad & 1) return g;
+        g.m = m;
+        g.q1 = h.bad == 0;
+        for (int k = 0; k < 10; ++k) g.row[k] = (double)h.ref[k];
+        return g;
+    }
+
+    EllGrid grid_check_result(const hb2_ell_s * A, const void * scratch)
+    {
+        const uint32_t m = grid_points(A);
+        if (! m) return EllGrid();
+        return A->dtype == HB2_F64 ? grid_result_typed<double>(m, scratch) : grid_result_typed<float>(m, scratch);
     }
 
     template <typename T>
