@@ -715,15 +715,17 @@ namespace
             {
                 const uint32_t r = perm[H * sl + j];
                 if (r == 0xffffffffu) continue;
-                auto & sp = span[sl / kWinWarps];
+                int32_t lo = INT32_MAX, hi = -1;
                 for (uint64_t k = 0; k < len(r); ++k)
                 {
                     const int32_t c = ecol[start[r] + k];
-                    sp.first = std::min(sp.first, c);
-                    sp.second = std::max(sp.second, c);
+                    lo = std::min(lo, c);
+                    hi = std::max(hi, c);
                     scol[slices[sl].x + H * k + j] = c;
                     sval[slices[sl].x + H * k + j] = eval[start[r] + k];
                 }
+                auto & sp = span[sl / kWinWarps];
+                sp = std::make_pair(std::min(sp.first, lo), std::max(sp.second, hi));
             }
         // each window's span of x; the staged kernel is a candidate when nine windows in ten fit
         // and the long rows are few enough for a CTA each
