@@ -333,7 +333,7 @@ namespace hb2
             if (red) HB2_CUDA(cudaMemsetAsync(red, 0, sizeof(double), stream));
             return HB2_OK;
         }
-        if (b.nvec == 1 && ! b.list && ! b.active && q1_single_applies(A, mode))
+        if (b.nvec == 1 && ! b.list && ! b.active && q1_single_applies(A, mode, red != 0))
         {
             if (red && ! ws) return fail(HB2_ERR_ARG, "fused reduction without a workspace");
             return launch_q1_single(A, mode, x, y, aux, red, want_sqrt, ws, stream);
@@ -986,7 +986,13 @@ extern "C" int hb2_jacobi_ell(hb2_ell A, const void * P, const void * b, void * 
     if (! A || ! P || ! b || ! x || (sweeps > 0 && ! tmp)) return fail(HB2_ERR_ARG, "hb2_jacobi_ell: null argument");
     if (A->rows != A->cols) return fail(HB2_ERR_SIZE, "hb2_jacobi_ell: needs a square matrix");
     // a Q1 grid operator: several sweeps a pass, in an even number of passes so that the
-    // result ends in x (one sweep: the plain pass below)
+    // result ends in x (one sweep: the plain pass below).  A pass of a single sweep has nothing to
+    // fuse and runs as the plain one where that is the faster: from 181 points a line, where the
+    // matrix leaves its plain arrays, in FP32 up to 1,000 points.  Two sweeps as passes of one / as
+    // plain ones (us, graphs of ten): FP64 6.3 / 9.0 at 181 points, 6.3 / 5.0 at 201, 8.4 / 6.3 at
+    // 513, 14.9 / 13.0 at 1,025, 62 / 52 at 2,049; FP32 7.3 / 5.8 at 513, 11.6 / 10.4 at 901,
+    // 11.7 / 11.8 at 1,001, 27.8 / 38.3 at 2,049.
+    const bool plain_one = A->layout[0] != kLayoutPlain && (A->dtype == HB2_F64 || A->q1g_m < 1000);
     if (A->q1g_m && sweeps >= 2)
     {
         uint64_t passes = (sweeps + kQ1SweepMax - 1) / kQ1SweepMax;
@@ -1002,7 +1008,8 @@ extern "C" int hb2_jacobi_ell(hb2_ell A, const void * P, const void * b, void * 
             p.b = b;
             p.jac = P;
             p.y = to;
-            const int st = launch_q1_sweep(A, p, stream);
+            const int st = p.sweeps == 1 && plain_one ? launch_ell(A, kJacobi, from, to, b, P, 0, 0, 0, 0, stream)
+                                                      : launch_q1_sweep(A, p, stream);
             if (st) return st;
             std::swap(from, to);
         }

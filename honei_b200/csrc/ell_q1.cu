@@ -734,7 +734,7 @@ namespace hb2
     int launch_ir_defect(const hb2_ell_s * A, const double * x, const double * b, float * b32, float * x32,
                          double * r64, double * red, const Workspace * ws, cudaStream_t stream)
     {
-        if (A->dtype == HB2_F64 && q1_single_applies(A, kDefect))
+        if (A->dtype == HB2_F64 && q1_single_applies(A, kDefect, true))
             return launch_q1_ir_defect(A, x, b, b32, x32, red, ws, stream);
         const uint64_t n = A->rows;
         const unsigned grid = ceil_div(n, kEllThreads);

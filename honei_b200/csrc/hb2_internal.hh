@@ -362,7 +362,7 @@ namespace hb2
     int launch_q1_sweep(const hb2_ell_s * A, const Q1SweepPass & p, cudaStream_t stream);
     // one product, defect or product with dot (kPlain, kDefect, kDot) as a streaming pass; the
     // refinement's outer defect (kDefectIR)
-    bool q1_single_applies(const hb2_ell_s * A, int mode);
+    bool q1_single_applies(const hb2_ell_s * A, int mode, bool reducing);
     int launch_q1_single(const hb2_ell_s * A, int mode, const void * x, void * y, const void * b, double * red,
                          int want_sqrt, const Workspace * ws, cudaStream_t stream);
     int launch_q1_ir_defect(const hb2_ell_s * A, const double * x, const double * b, float * b32, float * x32,

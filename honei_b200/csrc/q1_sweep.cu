@@ -151,12 +151,15 @@ namespace hb2
     }
 
     // Product, defect (+ norm) and product with dot of a large Q1 grid operator as streaming
-    // passes.  From 2^16 rows up: below, the one-row-per-thread kernels are as fast and their
-    // layout was timed at creation.  Measured (B200), FP64 level 11: defect + norm 37.2 us
-    // with the gather kernel, 26.6 as a streaming pass (a call, partial sums included).
-    bool q1_single_applies(const hb2_ell_s * A, int mode)
+    // passes; below, the row kernels, whose layout was timed at creation, are as fast or faster.
+    // Row kernel / streaming pass (B200, us, graphs of 20): product FP64 3.4 / 3.6 at 601 points a
+    // line, 4.4 / 4.3 at 801, 5.8 / 4.9 at 1,001, 19.2 / 12.2 at 2,049; defect FP64 5.3 / 5.8 at 901,
+    // 6.0 / 6.3 at 1,025, 6.9 / 6.5 at 1,101, FP32 5.0 / 5.1 at 901, 5.6 / 5.1 at 1,001; defect with
+    // its norm FP64 5.6 / 5.9 at 513, 6.7 / 6.3 at 601, 34.2 / 19.1 at 2,049 (FP32 the same lines).
+    bool q1_single_applies(const hb2_ell_s * A, int mode, bool reducing)
     {
-        return A->q1g_m >= 257 && (mode == kPlain || mode == kDefect || mode == kDot);
+        const uint32_t from = reducing ? 600 : mode == kPlain ? 768 : A->dtype == HB2_F64 ? 1100 : 950;
+        return A->q1g_m >= from && (mode == kPlain || mode == kDefect || mode == kDot);
     }
 
     int launch_q1_single(const hb2_ell_s * A, int mode, const void * x, void * y, const void * b, double * red,

@@ -44,6 +44,37 @@ def test_smoother_matches_single_sweeps(oracle, cells, npdt, sweeps):
     check_smoother(oracle, SparseMatrixELL.from_arrays(*op), ref, npdt, sweeps)
 
 
+# passes of one sweep beside passes of several: as sweep passes up to 181 points a line (the plain
+# layout) and, in FP32, from 1,000; as single sweeps between
+@pytest.mark.parametrize("cells", [180, 181, 998, 999])
+@pytest.mark.parametrize("npdt", [np.float64, np.float32])
+@pytest.mark.parametrize("sweeps", [2, 3])
+def test_smoother_with_passes_of_one_sweep(oracle, cells, npdt, sweeps):
+    op = q1_coefficient_operator(np.ones((cells, cells)), npdt)
+    check_smoother(oracle, SparseMatrixELL.from_arrays(*op), oracle_ell(oracle, op), npdt, sweeps)
+
+
+# either side of the sizes from which a product, a defect and a defect with its norm stream
+@pytest.mark.parametrize("cells", [598, 599, 766, 767, 948, 949, 1098, 1099])
+@pytest.mark.parametrize("npdt", [np.float64, np.float32])
+def test_single_passes(oracle, cells, npdt):
+    op = q1_coefficient_operator(np.ones((cells, cells)), npdt)
+    ref, A = oracle_ell(oracle, op), SparseMatrixELL.from_arrays(*op)
+    x, b = oracle.uniform(ref.rows, 3, npdt), oracle.uniform(ref.rows, 4, npdt)
+    xd, bd, y = dvec(x), dvec(b), dvec(np.zeros(ref.rows, npdt))
+    hb.Product.value(y, A, xd)
+    assert np.array_equal(y.numpy().view(np.uint8), oracle.ell_spmv(ref, x).view(np.uint8))
+    d = oracle.ell_defect(ref, b, x)
+    hb.Defect.value(y, bd, A, xd)
+    assert np.array_equal(y.numpy().view(np.uint8), d.view(np.uint8))
+    y, norm2 = dvec(np.zeros(ref.rows, npdt)), torch.zeros(1, dtype=torch.float64, device="cuda")
+    hb.Defect.value(y, bd, A, xd, norm2_out=norm2)
+    assert np.array_equal(y.numpy().view(np.uint8), d.view(np.uint8))
+    # a sum of n squares in FP64 in another order
+    exact = float(np.dot(d.astype(np.float64), d.astype(np.float64)))
+    assert abs(float(norm2) / exact - 1.0) <= ref.rows * 2.0 ** -52
+
+
 @pytest.mark.parametrize("npdt", [np.float64, np.float32])
 def test_smoother_anisotropic_operator(oracle, npdt):
     """Couplings that differ: the form with one product per slot."""
