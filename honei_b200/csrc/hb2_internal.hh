@@ -427,10 +427,6 @@ namespace hb2
         const void * jac;
     };
     constexpr uint64_t kSubMaxRows = 20000;
-    // levels that can run as sweep passes go into the cluster kernels only up to this many
-    // rows (a level-4 grid: whole level-6 solves 575 us with it there, 597 us without; the
-    // next larger grids are faster as sweep passes: 598 us with level 5 there, 668 with 5-6)
-    constexpr uint64_t kSubSweepRows = 300;
     int launch_subcycle(int dtype, const SubLevelDesc * lev, int top, int t1, int n_pre, int n_post, bool down,
                         cudaStream_t stream);
     int subcycle_prepare();

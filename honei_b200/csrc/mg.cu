@@ -25,7 +25,6 @@
 #include "hb2_common.cuh"
 #include "hb2_internal.hh"
 
-#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -614,7 +613,8 @@ namespace hb2
         int st = mg_alloc(mg, stream);
         if (st) return st;
         // the small levels (at most kSubMaxRows rows, above the coarsest) run as
-        // cluster kernels unless disabled
+        // cluster kernels unless disabled; levels that run as sweep passes do not, nor any
+        // level above a bottom block
         // (HB2_SUB_MAX_ROWS / HB2_SUB_LOCAL_ROWS override the two row limits;
         // HB2_SUB_FUSED=1 runs the small levels and the coarse CG as one launch,
         // measured slower on B200 than down / coarse CG / up as three)
@@ -639,12 +639,11 @@ namespace hb2
                 mg->bottom_top = (int)i;
             }
         const uint64_t max_rows = mg->bottom_top >= 1 ? 0 : env_u64("HB2_SUB_MAX_ROWS", kSubMaxRows);
-        const uint64_t sweep_rows = std::min<uint64_t>(max_rows, kSubSweepRows);
         const uint64_t local_rows = env_u64("HB2_SUB_LOCAL_ROWS", kSubLocalRows);
         if (! mg->prm.no_fused_levels && mg->prm.cycle == 0 && mg->prm.n_pre_smooth < (1u << 20) &&
             mg->prm.n_post_smooth < (1u << 20))
             for (uint32_t i = 1; i < mg->nlev && i < 10; ++i)
-                if (mg->lev[i].n <= (mg->lev[i].sweep ? sweep_rows : max_rows)) mg->sub_top = (int)i;
+                if (! mg->lev[i].sweep && mg->lev[i].n <= max_rows) mg->sub_top = (int)i;
         if (mg->sub_top >= 1)
         {
             for (int i = 1; i <= mg->sub_top; ++i)

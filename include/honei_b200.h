@@ -120,6 +120,10 @@ HB2_API int hb2_ell_info(hb2_ell A, uint64_t *rows, uint64_t *cols, uint64_t *st
  *                a table of *table_size patterns of (value, column - row) slots;
  *             3  BF16 values + 16-bit offsets or int32 columns (hb2_ell_create_bf16).
  * *row_bytes = matrix bytes read per row.  Every layout gives the same bits.
+ * Two kinds of square matrices, found at creation unless HB2_ELL_COMPACT pins a layout, have
+ * kernels that need no layout: Q1 grid operators with one set of values (large products and
+ * defects, several smoothing sweeps, multigrid levels, CG: the matrix is ten numbers) and
+ * nine-point grid matrices with any values on layout 0 (values read, columns not).
  * No counterpart in the reference (its device copy is the raw arrays). */
 HB2_API int hb2_ell_layout(hb2_ell A, int *layout, uint32_t *table_size, uint32_t *row_bytes);
 /* The kernel behind that choice, per kernel class (cls 0: products, sweeps and
@@ -381,8 +385,10 @@ typedef struct
     double coarse_eps;                      /* coarse CG eps (reference: = eps_relative) */
     double omega;                           /* Jacobi damping, 0.7 */
     int coarse_exact;                       /* 1: coarse CG dots in the reference's sequential fma order */
-    int no_fused_levels;                    /* 1: one kernel per operator on every level (0: levels below
-                                               ~20k rows run as two thread-block-cluster kernels per cycle) */
+    int no_fused_levels;                    /* 1: no launch spans several levels (0: the small levels of a
+                                               V-cycle share launches: up to 33 x 33 points with the coarse CG
+                                               in one block on Q1 grid hierarchies, else levels below ~20k
+                                               rows in two thread-block-cluster kernels per cycle) */
     int coarse_fp64;                        /* F32 hierarchies: 1 runs the coarsest CG in FP64 on an FP64 copy
                                                of the coarse operator (<= 128 rows, 1-9 slots); 0: FP32 as the reference */
     int cycle;                              /* 0: V-cycle (MGCycleCreation<V::STATIC>, math/mg.hh:567-656);

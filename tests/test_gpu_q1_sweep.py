@@ -140,3 +140,22 @@ def test_coarse_cg_on_the_grid(monkeypatch, coarse, aniso, cap, mixed):
     # each of the at most 24 sweeps and transfers of a cycle behind it.
     u = 2.0 ** -52 * 100 * 64 + (24 * 2.0 ** -23 if mixed else 0.0)
     assert np.abs(out[0] - out[1]).max() <= 2 * 2 * u * np.abs(out[1]).max()
+
+
+def test_coarsest_operator_with_more_slots(oracle):
+    """A coarsest matrix of ten slots (one of them empty) does not fit the bottom block: the levels
+    above run as sweep passes beside a coarse CG of their own.  Reference order, so the same bits."""
+    m = 33
+    i = torch.arange(m * m, device="cuda", dtype=torch.float64)
+    ref = oracle.q1_ell(3)
+    Aj, Ax = (np.concatenate([a, np.zeros(ref.stride, a.dtype)]) for a in (ref.Aj, ref.Ax))
+    wide = SparseMatrixELL.from_arrays(ref.rows, ref.cols, ref.stride, ref.K + 1, Aj, Ax, ref.Arl)
+    transfers = [SparseMatrixELL.transfer(level) for level in (4, 5)]
+    out = []
+    for coarse in (wide, SparseMatrixELL.poisson_q1(3)):
+        data = hb.MGData([coarse] + [SparseMatrixELL.poisson_q1(level) for level in (4, 5)], [t[0] for t in transfers],
+                         [t[1] for t in transfers], params=hb.mg_params(4, 4, max_iters=3, eps=1e-30, coarse_exact=True))
+        x = DenseVector(torch.cos(1.7 * i))
+        hb.MGSolver.value(data, DenseVector(torch.sin(i)), x)
+        out.append(x.numpy())
+    assert np.array_equal(out[0].view(np.uint8), out[1].view(np.uint8))
