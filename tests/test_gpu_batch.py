@@ -122,3 +122,26 @@ def test_bad_levels_are_rejected():
         hb.BatchedPoissonSolver([(4, 1)], coarse_level=4)
     with pytest.raises(_lib.HoneiError):
         hb.BatchedPoissonSolver([(2, 1)], coarse_level=3)
+
+
+# sweeps of the preconditioner other than four and four: more than a pass takes, in passes of
+# unequal length (5, 6, 9); an odd number of passes up, after which the result is copied back (1,
+# 2, 3, 9); different numbers each way
+@pytest.mark.parametrize("pre,post", [(1, 1), (2, 3), (3, 5), (5, 5), (6, 2), (4, 9), (9, 4)])
+def test_other_numbers_of_sweeps(oracle, monkeypatch, pre, post):
+    """Sweep passes against single passes, which every step clears the correction for: the same
+    bits, and each solution meets its tolerance."""
+    systems = [(4, 1), (6, 2), (7, 1)]
+    kw = {"params": hb.batch_params(eps=1e-8, n_pre=pre, n_post=post)}
+    out = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("HB2_Q1_TRANSFER", flag)       # 0: no transfer or sweep kernels
+        B, xs = solve_mix(systems, **kw)
+        out.append(xs)
+        for s, (level, k) in enumerate(systems):
+            A, b = oracle.q1_ell(level), rhs_for(s, level, k)
+            for j in range(k):
+                r = b[j] - oracle.ell_spmv(A, xs[s][j])
+                assert np.linalg.norm(r) <= 1.05e-8 * np.linalg.norm(b[j]), (s, j)
+    for a, c in zip(*out):
+        assert np.array_equal(a.view(np.uint8), c.view(np.uint8))

@@ -108,3 +108,43 @@ def test_cg_var_loop(oracle, cells, cap):
     s = hb.CGSmoother.value(A, dvec(P), dvec(b), dvec(np.zeros(n)), cap)
     so = oracle.cg_var(ref, P, b, max_iters=cap, eps=0.0, smoother=True)[0]
     assert np.linalg.norm(s.numpy() - so) <= 2.0 ** -52 * n * cap * np.linalg.norm(so)
+
+
+def loop_against_oracle(oracle, A, ref, cap):
+    n = ref.rows
+    P = oracle.jacobi_vector(ref)
+    b = oracle.ell_spmv(ref, uniform(n, 42))
+    x, used, _ = hb.KrylovSolver(hb.HB2_CG_VAR, A, dvec(P), cap, 0.0).solve(dvec(b), dvec(np.zeros(n)))
+    xo, ref_used = oracle.cg_var(ref, P, b, max_iters=cap, eps=0.0)[:2]
+    assert used == ref_used == cap
+    # as above: n eps a step, over `cap` steps
+    assert np.linalg.norm(x.numpy() - xo) <= 2.0 ** -52 * n * cap * np.linalg.norm(xo)
+
+
+# 5, 8, 9 and 13 rows a thread: either side of the instances' limits, and the largest that fits
+@pytest.mark.parametrize("cells", [600, 777, 800, 990])
+def test_cg_var_loop_with_many_rows_a_thread(oracle, cells):
+    op = q1_coefficient_operator(np.power(4.0, uniform(cells * cells, 5, -0.5, 0.5)).reshape(cells, cells))
+    ref = oracle.Ell(op[0], op[0], op[2], op[3], 1, *op[4:])
+    loop_against_oracle(oracle, SparseMatrixELL.from_arrays(*op), ref, 12)
+
+
+# a plain matrix that is no grid: nine slots unrolled, and any number of them (two more, empty);
+# 1, 2 and 5 rows a thread
+@pytest.mark.parametrize("cells", [50, 300, 600])
+@pytest.mark.parametrize("slots", [9, 11])
+def test_cg_var_loop_on_a_plain_matrix(oracle, monkeypatch, cells, slots):
+    monkeypatch.setenv("HB2_ELL_COMPACT", "0")       # the plain layout, and no look for grid operators
+    n, _, stride, K, Aj, Ax, Arl = q1_coefficient_operator(
+        np.power(4.0, uniform(cells * cells, 5, -0.5, 0.5)).reshape(cells, cells))
+    more = np.zeros((slots - K) * stride)
+    op = (n, n, stride, slots, np.concatenate([Aj, more.astype(Aj.dtype)]), np.concatenate([Ax, more]), Arl)
+    ref = oracle.Ell(n, n, stride, slots, 1, *op[4:])
+    loop_against_oracle(oracle, SparseMatrixELL.from_arrays(*op), ref, 12)
+
+
+# the constant-coefficient operator, whose matrix is ten numbers: 1, 4 and 14 rows a thread, the
+# last one beyond the loop's 13
+@pytest.mark.parametrize("level", [6, 9, 10])
+def test_cg_var_loop_on_the_constant_operator(oracle, level):
+    loop_against_oracle(oracle, SparseMatrixELL.poisson_q1(level), oracle.q1_ell(level), 12)
