@@ -1,7 +1,6 @@
 // Which matrices the Q1 sweep kernel (q1_sweep.cuh) serves, and its launch.
 #include "q1_sweep_impl.cuh"
 
-
 namespace hb2
 {
     int q1_sweep_f64(const Q1SweepArgs<double> & g, bool wide, bool uni, int S, int head, int tail, bool pvec,
@@ -129,7 +128,8 @@ namespace hb2
         // columns a lane.  FP64: two from level 9 (9.4 us a pass against 9.9 with one), one
         // below (level 8: 6.7 us), where a strip of 20 owned columns leaves more warps.  FP32:
         // four from level 11 (35.1 / 38.9 us down / up against 37.1 / 45.4 with two), two below
-        // (level 10: 11.9 / 15.3 us against 12.3 / 13.6; level 9: 6.9 / 9.4 against 8.5 / 9.9)
+        // (level 10: 11.9 / 15.3 us against 12.3 / 13.6; level 9: 6.9 / 9.4 against 8.5 / 9.9); the
+        // line between 1,025 and 2,049 points is not measured
         const bool wide = g.m >= (sizeof(T) == 8 ? 400 : 1500);
         if constexpr (sizeof(T) == 8)
             return q1_sweep_f64(g, wide, uni, p.sweeps, p.zero_guess ? kSweepZero : kSweepLoad, p.tail, p.pvec, l);

@@ -29,7 +29,7 @@
 // on the small grids the latency of a step times the rows of a chunk.  Measured (B200, graph
 // of 20 passes over vector sets larger than L2), FP64: the level-11 pass of four sweeps,
 // defect and restriction 49.8 us, of prolongation, four sweeps and norm 55.5 us, where the
-// single passes took about 165 and 155 us; level 10 15.5 / 18.6 us; FP32 level 11 35.4 us.
+// single passes took about 165 and 155 us; level 10 15.5 / 18.6 us; FP32 level 11 35.1 us.
 #pragma once
 
 #include "hb2_common.cuh"
@@ -240,7 +240,7 @@ namespace hb2
             constexpr int YLAG = NSM > 0 ? 2 * NSM - 1 : (sweep_single(TAIL) ? 1 : 0);
             T * yr = g.y + vo + col0 + ((int64_t)kb - YLAG) * m;
             const T * brl = bring + lane * C, * prl = pring + lane * C;
-                        auto step = [&](auto interior, auto parity, int s) {
+            auto step = [&](auto interior, auto parity, int s) {
                 constexpr bool IN = decltype(interior)::value;      // no boundary row in a stage
                 constexpr bool ODD = decltype(parity)::value;       // of s; the stages' rows have the other one
                 cp_async_wait<D - 1>();
@@ -491,6 +491,8 @@ namespace hb2
     // passes of levels 7 to 11: 0.29 us alone, 0.36 and 0.5 us; the model picks the fastest
     // or within 5 % of the fastest measured height at each level -- level 11: 48 rows 49.8 us
     // against 60.5 at 24 and 55.7 at 56; level 10: 20 rows 15.5 us, 12 rows 16.6, 40 rows 18.4).
+    // The FP32 passes, those with a given Jacobi vector and those without sweeps use the same step
+    // costs; theirs were not measured.
     inline int sweep_chunk_rows(int m, int strips, int halo, int ns, int per_sm, uint64_t nvec)
     {
         static const int cand[] = {2, 4, 6, 8, 10, 12, 16, 20, 24, 28, 32, 36, 40, 44, 48, 52, 56, 60, 64, 72, 80, 96,

@@ -55,7 +55,8 @@ class L2Flush:
 
 
 def graph_time(name, A, P, n, dt, npdt, dev, reps, launches=40):
-    """Mean time of one launch of `name` (jacobi / spmv / defect / copy) inside a CUDA
+    """Mean time of one launch of `name` (jacobi / spmv / defect / copy; sweeps: a smoother
+    call of eight sweeps, two passes of four on a Q1 grid operator) inside a CUDA
     graph of `launches` back-to-back launches that rotate over sets of input and
     output vectors (more than 2x L2 in all, so each launch reads its vectors from
     DRAM while the TLBs stay warm); CUDA events around each replay."""
@@ -77,6 +78,9 @@ def graph_time(name, A, P, n, dt, npdt, dev, reps, launches=40):
         if name == "jacobi":
             _lib.call("hb2_jacobi_sweep_ell", A.handle, ctypes.c_void_p(pj.data_ptr()), ctypes.c_void_p(b.data_ptr()),
                       ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(y.data_ptr()), st)
+        elif name == "sweeps":
+            _lib.call("hb2_jacobi_ell", A.handle, ctypes.c_void_p(pj.data_ptr()), ctypes.c_void_p(b.data_ptr()),
+                      ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(y.data_ptr()), 8, st)
         elif name == "spmv":
             _lib.call("hb2_product_ell", A.handle, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(y.data_ptr()), st)
         elif name == "defect":
