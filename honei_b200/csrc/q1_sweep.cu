@@ -153,12 +153,14 @@ namespace hb2
     // Product, defect (+ norm) and product with dot of a large Q1 grid operator as streaming
     // passes; below, the row kernels, whose layout was timed at creation, are as fast or faster.
     // Row kernel / streaming pass (B200, us, graphs of 20): product FP64 3.4 / 3.6 at 601 points a
-    // line, 4.4 / 4.3 at 801, 5.8 / 4.9 at 1,001, 19.2 / 12.2 at 2,049; defect FP64 5.3 / 5.8 at 901,
+    // line, 4.4 / 4.3 at 801, 5.8 / 4.9 at 1,001, 19.2 / 12.2 at 2,049, FP32 3.2 / 3.2 at 601,
+    // 3.7 / 3.3 at 701; defect FP64 5.3 / 5.8 at 901,
     // 6.0 / 6.3 at 1,025, 6.9 / 6.5 at 1,101, FP32 5.0 / 5.1 at 901, 5.6 / 5.1 at 1,001; defect with
     // its norm FP64 5.6 / 5.9 at 513, 6.7 / 6.3 at 601, 34.2 / 19.1 at 2,049 (FP32 the same lines).
     bool q1_single_applies(const hb2_ell_s * A, int mode, bool reducing)
     {
-        const uint32_t from = reducing ? 600 : mode == kPlain ? 768 : A->dtype == HB2_F64 ? 1100 : 950;
+        const bool f64 = A->dtype == HB2_F64;
+        const uint32_t from = reducing ? 600 : mode == kPlain ? (f64 ? 768 : 640) : f64 ? 1100 : 950;
         return A->q1g_m >= from && (mode == kPlain || mode == kDefect || mode == kDot);
     }
 

@@ -55,7 +55,7 @@ def test_smoother_with_passes_of_one_sweep(oracle, cells, npdt, sweeps):
 
 
 # either side of the sizes from which a product, a defect and a defect with its norm stream
-@pytest.mark.parametrize("cells", [598, 599, 766, 767, 948, 949, 1098, 1099])
+@pytest.mark.parametrize("cells", [598, 599, 638, 639, 766, 767, 948, 949, 1098, 1099])
 @pytest.mark.parametrize("npdt", [np.float64, np.float32])
 def test_single_passes(oracle, cells, npdt):
     op = q1_coefficient_operator(np.ones((cells, cells)), npdt)
